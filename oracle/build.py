@@ -36,7 +36,7 @@ def build_reference(ref_root=None):
     """Compile parts of the reference in place (only where the tree exists):
     its key codecs, geometry placement and regrid/hash kernels."""
     ref_root = ref_root or REF_ROOT
-    if not os.path.isdir(ref_root):
+    if not os.path.isdir(os.path.join(ref_root, "src")):  # absent, or an empty mount point
         return None
     subprocess.run(["make", "-s", "-f", os.path.join(HERE, "Makefile.ref"), "REF=" + ref_root],
                    check=True)
