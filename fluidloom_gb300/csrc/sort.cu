@@ -15,17 +15,20 @@
 //     writes it out with coalesced runs.
 // Four shapes, chosen per context (fl_sort_set_config): 8- or 9-bit digits (9:
 // 7 passes over 63-bit keys instead of 8) on tiles of 256 or 512 threads x 12
-// keys (512: half the tiles and twice the keys per digit run written, at 2
-// CTAs per SM; 256: 4 CTAs per SM with 8-bit digits, 3 with 9-bit, whose
-// threads then take two digits each).
+// keys, or x 4 for up to kSmallSort keys (512: half the tiles and twice the
+// keys per digit run written, at 2 CTAs per SM; 256: 4 CTAs per SM with 8-bit
+// digits, 3 with 9-bit, whose threads then take two digits each).
 // Stable: ties keep input order, so (key, payload) pairs match std::stable_sort.
 #include "common.cuh"
 #include "scan.cuh"
 
+#include <type_traits>
+
 namespace {
 
-constexpr int kItems = 12;                 // keys per thread in a tile
-constexpr int kTileMin = 256 * kItems;     // the smallest tile: scratch is sized for it
+constexpr int kLargeItems = 12;            // keys per thread in a tile
+constexpr int kSmallItems = 4;             // ... of a small sort
+constexpr int kSmallWindow = 4;            // predecessors a small sort's look-back reads at once
 constexpr int kMaxRadix = 512;
 constexpr int kMaxPasses = 8;              // 64-bit keys, 8- or 9-bit digits
 
@@ -83,13 +86,13 @@ __device__ __forceinline__ uint32_t ld_vol(const uint32_t* p) { return *(volatil
 // Dynamic shared memory of one onesweep tile: keys and values staged in rank
 // order, per-warp digit counters, per-digit tile offsets and global bases,
 // per-warp sums of the digit scan.
-template <int kThreads, int kBits>
+template <int kThreads, int kBits, int kItems>
 __host__ __device__ constexpr size_t onesweep_smem() {
     return (size_t)kThreads * kItems * 12 +
            ((size_t)(kThreads / 32) * (1 << kBits) + 2 * (1 << kBits) + kThreads / 32) * 4;
 }
 
-template <int kThreads, int kBits>
+template <int kThreads, int kBits, int kItems>
 __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 4 : 3))
     k_onesweep(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
                uint32_t* __restrict__ vout, size_t n, int shift, uint32_t dmask,
@@ -158,19 +161,47 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
             *(volatile uint32_t*)st = kFlagAgg | run;
             int t = tile - 1;
             unsigned spins = 0;
-            while (t >= 0) {
-                uint32_t s = ld_vol(status + (size_t)t * R + d);
-                if ((s & kFlagMask) == 0) {
-                    if (++spins > FL_SPIN_LIMIT) {
+            if constexpr (kItems == kSmallItems) {
+                // kSmallWindow predecessors per round trip, the nearest first; tile 0 publishes
+                // an inclusive word, so the walk ends there at the latest
+                bool found = false;
+                while (!found) {
+                    uint32_t s[kSmallWindow];
+#pragma unroll
+                    for (int j = 0; j < kSmallWindow; ++j)
+                        s[j] = t >= j ? ld_vol(status + (size_t)(t - j) * R + d) : 0u;
+                    int used = 0;
+                    bool ready = true;
+#pragma unroll
+                    for (int j = 0; j < kSmallWindow; ++j) {
+                        ready = ready && !found && (s[j] & kFlagMask) != 0;
+                        if (!ready) continue;
+                        prefix += s[j] & kValMask;
+                        found = (s[j] & kFlagMask) == kFlagInc;
+                        ++used;
+                    }
+                    t -= used;
+                    if (used == 0 && ++spins > FL_SPIN_LIMIT) {
                         atomicAdd(dev_status + FL_DEVSTAT_TIMEOUT, 1u);
                         s_bad = 1;
                         break;
                     }
-                    continue;
                 }
-                prefix += s & kValMask;
-                if ((s & kFlagMask) == kFlagInc) break;
-                --t;
+            } else {
+                while (t >= 0) {
+                    uint32_t s = ld_vol(status + (size_t)t * R + d);
+                    if ((s & kFlagMask) == 0) {
+                        if (++spins > FL_SPIN_LIMIT) {
+                            atomicAdd(dev_status + FL_DEVSTAT_TIMEOUT, 1u);
+                            s_bad = 1;
+                            break;
+                        }
+                        continue;
+                    }
+                    prefix += s & kValMask;
+                    if ((s & kFlagMask) == kFlagInc) break;
+                    --t;
+                }
             }
             *(volatile uint32_t*)st = kFlagInc | ((prefix + run) & kValMask);
         }
@@ -233,18 +264,27 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
     }
 }
 
+// A pass of one tile is a chain of latencies (about 11,800 cycles at 12 keys per thread: 4,000 rank
+// them, 1,800 stage them, 2,400 write them out), so while the tiles fit the GPU at once a sort takes
+// as long as one tile, and fewer keys per thread make more and shorter tiles.  Their look-back is
+// longer, so it reads kSmallWindow words per round trip.  Keys and sort, 12 -> 4 keys per thread:
+// 3,000 63-bit keys 84 -> 65 us, 40,961 30-bit keys 61 -> 51, 240,000 63-bit keys 128 -> 120,
+// 600,000 162 -> 158; at 1,000,000 the tiles no longer fit at once, 196 -> 214.
+constexpr size_t kSmallSort = 1u << 19;
+
 // Bytes of one pass's tile status words and ticket, for every shape: at most
-// ceil(n / kTileMin) tiles of at most kMaxRadix digits (9-bit digits on the
+// ceil(n / smallest tile) tiles of at most kMaxRadix digits (9-bit digits on the
 // smallest tile reach both bounds at once).
 size_t status_stride_min(size_t n) {
-    return fl_align256(((n + kTileMin - 1) / kTileMin) * kMaxRadix * 4 + 4) + 4096;
+    const size_t tile = 256 * (n <= kSmallSort ? kSmallItems : kLargeItems);
+    return fl_align256(((n + tile - 1) / tile) * kMaxRadix * 4 + 4) + 4096;
 }
 
 // All passes of one shape.  The scratch layout (fl_sort_scratch_bytes): the
 // alternate key and value buffers, the pass histograms (kMaxPasses x
 // kMaxRadix), then per pass its tile status words and ticket, at a stride that
 // fits every shape's tiles (status_stride_min).
-template <int kThreads, int kBits>
+template <int kThreads, int kBits, int kItems>
 int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit, void* scratch) {
     constexpr int R = 1 << kBits;
     constexpr int kTile = kThreads * kItems;
@@ -256,12 +296,12 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
     uint32_t* valt = (uint32_t*)p; p += fl_align256(n * 4);
     uint32_t* hist = (uint32_t*)p; p += fl_align256((size_t)kMaxPasses * kMaxRadix * 4);
     char* stat0 = p;
-    const size_t stat_stride = status_stride_min(n);
+    const size_t stat_stride = fl_align256(tiles * R * 4 + 4);  // at most status_stride_min(n)
     // clear histograms + per-pass status/tickets in one memset
     FL_TRY_CUDA(ctx, cudaMemsetAsync(hist, 0, fl_align256((size_t)kMaxPasses * kMaxRadix * 4) + passes * stat_stride,
                                      ctx->stream), "sort clear");
-    constexpr size_t smem = onesweep_smem<kThreads, kBits>();
-    FL_TRY_CUDA(ctx, cudaFuncSetAttribute(k_onesweep<kThreads, kBits>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    constexpr size_t smem = onesweep_smem<kThreads, kBits, kItems>();
+    FL_TRY_CUDA(ctx, cudaFuncSetAttribute(k_onesweep<kThreads, kBits, kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem), "sort shared memory");
     unsigned hb = fl_blocks(n, 256, ctx->num_sms * 4);
     k_histogram<kBits><<<hb, 256, 0, ctx->stream>>>(keys, n, begin_bit, end_bit, passes, hist);
@@ -275,7 +315,7 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
         uint32_t* status = (uint32_t*)(stat0 + ps * stat_stride);
         unsigned* ticket = (unsigned*)(status + tiles * R);
         int sh = begin_bit + kBits * ps;
-        k_onesweep<kThreads, kBits><<<(unsigned)tiles, kThreads, smem, ctx->stream>>>(
+        k_onesweep<kThreads, kBits, kItems><<<(unsigned)tiles, kThreads, smem, ctx->stream>>>(
             ks[cur], vs[cur], ks[cur ^ 1], vs[cur ^ 1], n, sh, digit_mask(end_bit, sh, kBits), hist + ps * R, status,
             ticket, ctx->dev_status);
         FL_CHECK_LAUNCH(ctx, "k_onesweep");
@@ -299,11 +339,16 @@ size_t fl_sort_scratch_bytes(size_t n, int passes) {
 int fl_sort_pairs_with(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit,
                        void* scratch) {
     if (n <= 1 || end_bit <= begin_bit) return FL_OK;
-    if (ctx->sort_digit_bits == 9 && ctx->sort_tile_threads == 256)
-        return sort_passes<256, 9>(ctx, keys, vals, n, begin_bit, end_bit, scratch);
-    if (ctx->sort_digit_bits == 9) return sort_passes<512, 9>(ctx, keys, vals, n, begin_bit, end_bit, scratch);
-    if (ctx->sort_tile_threads == 512) return sort_passes<512, 8>(ctx, keys, vals, n, begin_bit, end_bit, scratch);
-    return sort_passes<256, 8>(ctx, keys, vals, n, begin_bit, end_bit, scratch);
+    const bool wide = ctx->sort_tile_threads == 512, nine = ctx->sort_digit_bits == 9;
+    auto run = [&](auto items) {
+        constexpr int I = decltype(items)::value;
+        if (nine)
+            return wide ? sort_passes<512, 9, I>(ctx, keys, vals, n, begin_bit, end_bit, scratch)
+                        : sort_passes<256, 9, I>(ctx, keys, vals, n, begin_bit, end_bit, scratch);
+        return wide ? sort_passes<512, 8, I>(ctx, keys, vals, n, begin_bit, end_bit, scratch)
+                    : sort_passes<256, 8, I>(ctx, keys, vals, n, begin_bit, end_bit, scratch);
+    };
+    return n <= kSmallSort ? run(std::integral_constant<int, kSmallItems>()) : run(std::integral_constant<int, kLargeItems>());
 }
 
 extern "C" int fl_sort_set_config(fl_ctx* ctx, int digit_bits, int tile_threads) {
