@@ -708,7 +708,7 @@ static size_t fl_balance_act_bytes(size_t n) { return fl_align256(n) + fl_align2
 size_t fl_adapt_scratch_bytes(size_t n, uint64_t cap) {
     size_t b = 0;
     b += fl_align256(n * 8);                 // cell keys (FACE6's hash table)
-    b += fl_align256(cap * 16) + fl_align256(cap * 4);  // 16-byte-slot table + win
+    b += fl_align256(cap * 16);              // 16-byte-slot table
     b += 2 * fl_align256(n) + fl_balance_act_bytes(n);  // shadow, viol, probing leaves
     b += 4 * fl_align256(n * 4);             // leader, gid, group_of, cnt/off
     b += fl_align256(n * 4);                 // members (n/8 groups * 8)
@@ -795,7 +795,7 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
 // Scratch layout of one regrid (carved identically by both phases).
 struct AdaptWork {
     uint64_t cap;
-    uint64_t* keys; uint64_t* tk; uint32_t* tv; uint32_t* win;
+    uint64_t* keys; uint64_t* tk; uint32_t* tv;
     uint8_t* shadow; uint8_t* viol; uint8_t* act;
     uint32_t* leader; uint32_t* gid; uint32_t* group_of; uint32_t* cnt; uint32_t* members; uint32_t* counters;
     void* scan_scratch;
@@ -809,7 +809,6 @@ static AdaptWork carve_adapt(void* scratch, size_t n, bool with_case) {
     w.keys = cv.take<uint64_t>(n);
     w.tk = cv.take<uint64_t>(2 * w.cap);
     w.tv = nullptr;  // 16-byte slots
-    w.win = cv.take<uint32_t>(w.cap);
     w.shadow = cv.take<uint8_t>(n);
     w.viol = cv.take<uint8_t>(n);
     w.act = cv.take<uint8_t>(fl_balance_act_bytes(n));
@@ -856,7 +855,7 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
         rc = fl_launch_cell_keys(ctx, mesh->x, mesh->y, mesh->z, mesh->level, mesh->case_id, dom.depth,
                                  dom.anchor_level, w.keys, n);
         if (rc) return rc;
-        rc = fl_hash_build_with(ctx, w.tk, w.tv, w.cap, w.keys, nullptr, n, w.win, mesh->level);  // level | index
+        rc = fl_hash_build_with(ctx, w.tk, w.tv, w.cap, w.keys, nullptr, n, mesh->level);  // level | index
         if (rc) return rc;
     }
     FL_TRY_CUDA(ctx, cudaMemsetAsync(w.counters, 0, 64, ctx->stream), "adapt counters");
@@ -962,7 +961,7 @@ int fl_balance_enforce(fl_ctx* ctx, fl_mesh* mesh, const fl_adapt_config* cfg, f
     if (n == 0) { if (res) res->converged = 1; return FL_OK; }
     const bool face6 = cfg->balance_mode == 0;  // FACE6 probes shadow levels through the hash table
     uint64_t cap = face6 ? fl_table_capacity(n) : 0;
-    size_t need = fl_align256(n * 8) + fl_align256(cap * 16) + fl_align256(cap * 4) + 2 * fl_align256(n) +
+    size_t need = fl_align256(n * 8) + fl_align256(cap * 16) + 2 * fl_align256(n) +
                   fl_balance_act_bytes(n) + 512 + 256 +
                   (face6 ? 0 : fl_locator_scratch_bytes(n));
     int rc = fl_scratch_reserve(ctx, need);
@@ -972,7 +971,6 @@ int fl_balance_enforce(fl_ctx* ctx, fl_mesh* mesh, const fl_adapt_config* cfg, f
     uint64_t* keys = cv.take<uint64_t>(n);
     uint64_t* tk = cv.take<uint64_t>(2 * cap);
     uint32_t* tv = nullptr;  // 16-byte slots
-    uint32_t* win = cv.take<uint32_t>(cap);
     uint8_t* shadow = cv.take<uint8_t>(n);
     uint8_t* viol = cv.take<uint8_t>(n);
     uint8_t* act = cv.take<uint8_t>(fl_balance_act_bytes(n));
@@ -984,7 +982,7 @@ int fl_balance_enforce(fl_ctx* ctx, fl_mesh* mesh, const fl_adapt_config* cfg, f
         rc = fl_launch_cell_keys(ctx, mesh->x, mesh->y, mesh->z, mesh->level, mesh->case_id, dom.depth,
                                  dom.anchor_level, keys, n);
         if (rc) return rc;
-        rc = fl_hash_build_with(ctx, tk, tv, cap, keys, nullptr, n, win, mesh->level);
+        rc = fl_hash_build_with(ctx, tk, tv, cap, keys, nullptr, n, mesh->level);
     } else {
         rc = fl_locator_build(ctx, md, dom, cv.p, &L);
     }

@@ -5,9 +5,9 @@
 // which launch nothing) with the kernels they name (kernels/hashmap/hash_build.cl:19-82,
 // kernels/hashmap/hash_query.cl:22-98): EMPTY key = ~0, INVALID value = ~0,
 // power-of-two capacity, linear probing, a repeated key keeps the value of
-// the LAST input carrying it (the order sequential insertion gives; resolved,
-// only when a build meets repeated keys, with an atomicMax on the input index
-// so the result does not depend on thread timing).  The slot is the high bits of key * 0x9e3779b97f4a7c15
+// the LAST input carrying it (the order sequential insertion gives; resolved
+// with an atomicMax on the input index, in the API's tables only when a build
+// meets repeated keys, so the result does not depend on thread timing).  The slot is the high bits of key * 0x9e3779b97f4a7c15
 // (Fibonacci hashing); the reference masks the low bits, which for 12-state
 // keys of coarse anchors fall on a handful of slots.
 #include "common.cuh"
@@ -26,7 +26,7 @@ __global__ void k_hash_clear(uint64_t* __restrict__ tk, uint32_t* __restrict__ t
             tk[i] = FL_EMPTY_KEY;
             tv[i] = FL_INVALID_INDEX;
         } else {
-            reinterpret_cast<ulonglong2*>(tk)[i] = make_ulonglong2(FL_EMPTY_KEY, FL_INVALID_INDEX);
+            reinterpret_cast<ulonglong2*>(tk)[i] = make_ulonglong2(FL_EMPTY_KEY, 0ull);
         }
     }
 }
@@ -39,61 +39,52 @@ __device__ __forceinline__ uint32_t hash_value_of(size_t i, const uint32_t* __re
     return (uint32_t)i;
 }
 
-__device__ __forceinline__ void hash_store_value(uint64_t* tk, uint32_t* tv, uint64_t s, uint32_t v) {
-    if (tv) tv[s] = v;
-    else tk[2 * s + 1] = v;
+// Insertion into the 16-byte-slot layout: the slot's key word by CAS, its value word by a 64-bit
+// maximum of (input index + 1) << 32 | value, so a repeated key ends with the value of its last
+// input whatever the order of the threads.
+__device__ __forceinline__ void hash_store_max(uint64_t* tk, uint64_t s, size_t i, uint32_t v) {
+    atomicMax((unsigned long long*)(tk + 2 * s + 1), ((unsigned long long)(i + 1) << 32) | v);
 }
 
-// Insertion: the thread whose CAS claims an empty slot stores its value with a
-// plain store; a thread that finds its key already there flags the build
-// (FL_DEVSTAT_HASH_DUPS) and stores nothing.  Without repeated keys that is
-// the table; with them the three passes below give each repeated key the
-// value of its last input.
-__global__ void k_hash_insert(uint64_t* __restrict__ tk, uint32_t* __restrict__ tv, int lg,
-                              const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals,
-                              const uint8_t* __restrict__ levels, size_t n, uint32_t* dev_status) {
+// Insertion into separate key and value arrays: the thread whose CAS claims an empty slot stores
+// its value with a plain store; a thread that finds its key already there flags the build
+// (FL_DEVSTAT_HASH_DUPS) and stores nothing.  Without repeated keys that is the table; with them
+// the three passes below give each repeated key the value of its last input.
+template <bool kPacked>
+__global__ void __launch_bounds__(256) k_hash_insert(uint64_t* __restrict__ tk, uint32_t* __restrict__ tv, int lg,
+                                                     const uint64_t* __restrict__ keys,
+                                                     const uint32_t* __restrict__ vals,
+                                                     const uint8_t* __restrict__ levels, size_t n,
+                                                     uint32_t* dev_status) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const uint64_t mask = (1ull << lg) - 1;
-    const int sw = tv ? 1 : 2;
-    for (size_t base = (size_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-        const size_t i = base + threadIdx.x;
-        bool dup = false;
-        if (i < n) {
-            const uint64_t k = keys[i];
-            if (k != FL_EMPTY_KEY) {
-                uint64_t s = fl_hash_slot(k, lg);
-                int p = 0;
-                for (; p < kProbeLimit; ++p) {
-                    unsigned long long prev = atomicCAS((unsigned long long*)(tk + s * sw), FL_EMPTY_KEY, k);
-                    if (prev == FL_EMPTY_KEY) {
-                        hash_store_value(tk, tv, s, hash_value_of(i, vals, levels));
-                        break;
-                    }
-                    if (prev == k) {
-                        dup = true;
-                        break;
-                    }
-                    s = (s + 1) & mask;
-                }
-                if (p == kProbeLimit) atomicAdd(dev_status + FL_DEVSTAT_HASH_OVERFLOW, 1u);
+    constexpr int sw = kPacked ? 2 : 1;
+    bool dup = false;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint64_t k = keys[i];
+        if (k == FL_EMPTY_KEY) continue;
+        uint64_t s = fl_hash_slot(k, lg);
+        int p = 0;
+        for (; p < kProbeLimit; ++p) {
+            const unsigned long long prev = atomicCAS((unsigned long long*)(tk + s * sw), FL_EMPTY_KEY, k);
+            if (prev == FL_EMPTY_KEY || prev == k) {
+                if (kPacked) hash_store_max(tk, s, i, hash_value_of(i, vals, levels));
+                else if (prev == FL_EMPTY_KEY) tv[s] = hash_value_of(i, vals, levels);
+                else dup = true;
+                break;
             }
+            s = (s + 1) & mask;
         }
-        if (__any_sync(0xFFFFFFFFu, dup) && (threadIdx.x & 31) == 0) atomicOr(dev_status + FL_DEVSTAT_HASH_DUPS, 1u);
+        if (p == kProbeLimit) atomicAdd(dev_status + FL_DEVSTAT_HASH_OVERFLOW, 1u);
     }
+    if (!kPacked && dup) atomicOr(dev_status + FL_DEVSTAT_HASH_DUPS, 1u);
 }
 
-// Repeated keys only (each kernel returns at once when the build met none):
-// clear the winner words, let every input take the maximum of its slot's
-// winner (input index + 1), then store each claimed slot's winning value.
-__global__ void k_hash_dup_clear(uint32_t* __restrict__ win, uint64_t cap, const uint32_t* dev_status) {
-    if (!*(volatile const uint32_t*)(dev_status + FL_DEVSTAT_HASH_DUPS)) return;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += stride) win[i] = 0u;
-}
-
-__global__ void k_hash_dup_winners(const uint64_t* __restrict__ tk, int sw, uint32_t* __restrict__ win, int lg,
-                                   const uint64_t* __restrict__ keys, size_t n, const uint32_t* dev_status) {
-    if (!*(volatile const uint32_t*)(dev_status + FL_DEVSTAT_HASH_DUPS)) return;
+// Repeated keys only, launched when a build into separate arrays met some (three launches that
+// returned at once in every other build took 11 us): every input takes the maximum of its slot's
+// winner (input index + 1), then each claimed slot gets its winning value.
+__global__ void k_hash_dup_winners(const uint64_t* __restrict__ tk, uint32_t* __restrict__ win, int lg,
+                                   const uint64_t* __restrict__ keys, size_t n) {
     size_t stride = (size_t)gridDim.x * blockDim.x;
     const uint64_t mask = (1ull << lg) - 1;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -101,7 +92,7 @@ __global__ void k_hash_dup_winners(const uint64_t* __restrict__ tk, int sw, uint
         if (k == FL_EMPTY_KEY) continue;
         uint64_t s = fl_hash_slot(k, lg);
         for (int p = 0; p < kProbeLimit; ++p) {
-            const uint64_t cur = tk[s * sw];
+            const uint64_t cur = tk[s];
             if (cur == k) {
                 atomicMax(win + s, (uint32_t)(i + 1));
                 break;
@@ -112,14 +103,12 @@ __global__ void k_hash_dup_winners(const uint64_t* __restrict__ tk, int sw, uint
     }
 }
 
-__global__ void k_hash_dup_values(uint64_t* __restrict__ tk, uint32_t* __restrict__ tv,
-                                  const uint32_t* __restrict__ win, const uint32_t* __restrict__ vals,
-                                  const uint8_t* __restrict__ levels, uint64_t cap, const uint32_t* dev_status) {
-    if (!*(volatile const uint32_t*)(dev_status + FL_DEVSTAT_HASH_DUPS)) return;
+__global__ void k_hash_dup_values(uint32_t* __restrict__ tv, const uint32_t* __restrict__ win,
+                                  const uint32_t* __restrict__ vals, uint64_t cap) {
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += stride) {
         const uint32_t w = win[i];
-        if (w) hash_store_value(tk, tv, i, hash_value_of(w - 1, vals, levels));
+        if (w) tv[i] = hash_value_of(w - 1, vals, nullptr);
     }
 }
 
@@ -346,7 +335,7 @@ int fl_hash_lg(uint64_t cap) {
 }
 
 int fl_hash_build_with(fl_ctx* ctx, uint64_t* tk, uint32_t* tv, uint64_t cap, const uint64_t* keys,
-                       const uint32_t* vals, size_t n, uint32_t* win, const uint8_t* levels) {
+                       const uint32_t* vals, size_t n, const uint8_t* levels) {
     if (levels && !vals && n >= ((size_t)1 << kPackedIdxBits))
         return fl_set_error(ctx, FL_E_CAPACITY, "a mesh of 2^27 or more cells");
     unsigned cb = fl_blocks(cap, 256, ctx->num_sms * 8);
@@ -354,17 +343,11 @@ int fl_hash_build_with(fl_ctx* ctx, uint64_t* tk, uint32_t* tv, uint64_t cap, co
     FL_CHECK_LAUNCH(ctx, "k_hash_clear");
     if (n == 0) return FL_OK;
     const uint8_t* lv = vals ? nullptr : levels;
-    FL_TRY_CUDA(ctx, cudaMemsetAsync(ctx->dev_status + FL_DEVSTAT_HASH_DUPS, 0, 4, ctx->stream), "hash flag");
     int lg = fl_hash_lg(cap);
     unsigned nb = fl_blocks(n, 256, ctx->num_sms * 8);
-    k_hash_insert<<<nb, 256, 0, ctx->stream>>>(tk, tv, lg, keys, vals, lv, n, ctx->dev_status);
+    if (tv) k_hash_insert<false><<<nb, 256, 0, ctx->stream>>>(tk, tv, lg, keys, vals, lv, n, ctx->dev_status);
+    else k_hash_insert<true><<<nb, 256, 0, ctx->stream>>>(tk, nullptr, lg, keys, vals, lv, n, ctx->dev_status);
     FL_CHECK_LAUNCH(ctx, "k_hash_insert");
-    k_hash_dup_clear<<<cb, 256, 0, ctx->stream>>>(win, cap, ctx->dev_status);
-    FL_CHECK_LAUNCH(ctx, "k_hash_dup_clear");
-    k_hash_dup_winners<<<nb, 256, 0, ctx->stream>>>(tk, tv ? 1 : 2, win, lg, keys, n, ctx->dev_status);
-    FL_CHECK_LAUNCH(ctx, "k_hash_dup_winners");
-    k_hash_dup_values<<<cb, 256, 0, ctx->stream>>>(tk, tv, win, vals, lv, cap, ctx->dev_status);
-    FL_CHECK_LAUNCH(ctx, "k_hash_dup_values");
     return FL_OK;
 }
 
@@ -392,10 +375,21 @@ int fl_hash_build(fl_ctx* ctx, uint64_t* table_keys, uint32_t* table_vals, uint6
     if (!table_keys || !table_vals || capacity == 0 || (capacity & (capacity - 1)) || (n && !keys))
         return fl_set_error(ctx, FL_E_INVALID_ARG, "fl_hash_build: bad table or capacity not a power of two");
     if (n > capacity) return fl_set_error(ctx, FL_E_CAPACITY, "fl_hash_build: more keys than slots");
-    int rc = fl_scratch_reserve(ctx, capacity * 4);
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(ctx->dev_status + FL_DEVSTAT_HASH_DUPS, 0, 4, ctx->stream), "hash flag");
+    int rc = fl_hash_build_with(ctx, table_keys, table_vals, capacity, keys, vals, n);
     if (rc) return rc;
-    rc = fl_hash_build_with(ctx, table_keys, table_vals, capacity, keys, vals, n, (uint32_t*)ctx->scratch);
+    rc = fl_collect_device_status(ctx, "fl_hash_build");
+    if (rc || !ctx->host_status[FL_DEVSTAT_HASH_DUPS]) return rc;
+    // repeated keys: the winner of each slot in a second round
+    rc = fl_scratch_reserve(ctx, capacity * 4);
     if (rc) return rc;
+    uint32_t* win = (uint32_t*)ctx->scratch;
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(win, 0, capacity * 4, ctx->stream), "hash winners");
+    k_hash_dup_winners<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(table_keys, win,
+                                                                                    fl_hash_lg(capacity), keys, n);
+    FL_CHECK_LAUNCH(ctx, "k_hash_dup_winners");
+    k_hash_dup_values<<<fl_blocks(capacity, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(table_vals, win, vals, capacity);
+    FL_CHECK_LAUNCH(ctx, "k_hash_dup_values");
     return fl_collect_device_status(ctx, "fl_hash_build");
 }
 

@@ -35,8 +35,8 @@ static __device__ __forceinline__ uint64_t fl_hash_slot(uint64_t key, int lg) {
 
 // Two layouts: the API tables keep keys and values in separate arrays (tk, tv,
 // HashTableManager's getKeysDevicePtr / getValuesDevicePtr); the tables the
-// library builds for itself store each slot as 16 bytes -- key, value, padding
-// -- so one probe reads one 32-byte sector instead of two.  tv == nullptr marks
+// library builds for itself store each slot as 16 bytes -- key, then (input
+// index + 1) << 32 | value -- so one probe reads one 32-byte sector instead of two.  tv == nullptr marks
 // such a table, tk then pointing at 2 * capacity words.
 // hash_query (kernels/hashmap/hash_query.cl:22-56) with the slot rule above.
 static __device__ __forceinline__ uint32_t fl_hash_lookup(const uint64_t* __restrict__ tk,
@@ -234,8 +234,10 @@ int fl_neighbours_sorted(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev&
 
 int fl_hash_lg(uint64_t cap);
 uint64_t fl_table_capacity(size_t n);
-// Clear + build; `win` is cap uint32 of scratch; tv == nullptr builds the
-// 16-byte-slot layout in tk (2 * cap words).  With `levels` (and no vals) the
-// values are levels[i] << 27 | i (n < 2^27, else FL_E_CAPACITY).
+// Clear + build; tv == nullptr builds the 16-byte-slot layout in tk (2 * cap
+// words; a repeated key keeps the value of its last input), else the API's
+// arrays, where a build that met repeated keys sets FL_DEVSTAT_HASH_DUPS and
+// leaves them to the caller.  With `levels` (and no vals) the values are
+// levels[i] << 27 | i (n < 2^27, else FL_E_CAPACITY).
 int fl_hash_build_with(fl_ctx* ctx, uint64_t* tk, uint32_t* tv, uint64_t cap, const uint64_t* keys,
-                       const uint32_t* vals, size_t n, uint32_t* win, const uint8_t* levels = nullptr);
+                       const uint32_t* vals, size_t n, const uint8_t* levels = nullptr);
