@@ -40,8 +40,8 @@ namespace {
 constexpr int kT = 256;
 
 struct KeyTables {
-    uint8_t t1[96];
-    uint16_t t3[12 * 512];
+    alignas(16) uint8_t t1[96];
+    alignas(16) uint16_t t3[12 * 512];
 };
 
 __device__ __forceinline__ bool fold3(int64_t* p, const fl_domain_dev::Case& d, int A) {
@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(kDetectThreads, 3) k_detect_full26(fl_mesh_dev
                                                                      uint8_t* __restrict__ nxt,
                                                                      uint8_t* __restrict__ viol,
                                                                      uint32_t* __restrict__ count) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     __shared__ uint8_t s_dir[8][19];  // per child position (x&1 | (y&1)<<1 | (z&1)<<2): outward directions
     fl_keys_fill_tables_cat(t1, t3c);
     if (threadIdx.x < 8) {
@@ -317,8 +317,8 @@ __device__ __forceinline__ uint32_t sibling_in_run(const fl_probe& P, const fl_m
 __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom, fl_locator L, int min_level,
                                                 int check26, const uint8_t* __restrict__ shadow,
                                                 uint32_t* __restrict__ is_leader) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     __shared__ uint8_t surf[56];  // the outside cells k = ux + 4 uy + 16 uz of the 4^3 grid of child-sized cells
     fl_keys_fill_tables_cat(t1, t3c);
     if (threadIdx.x == 0) {
@@ -425,8 +425,8 @@ __global__ void __launch_bounds__(kT) k_members(fl_mesh_dev m, fl_domain_dev dom
                                                 const uint32_t* __restrict__ is_leader,
                                                 const uint32_t* __restrict__ gid, uint32_t* __restrict__ members,
                                                 uint32_t* __restrict__ group_of) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();
     const fl_probe P = fl_probe_make(t1, t3c, L, dom);
@@ -495,8 +495,8 @@ __global__ void __launch_bounds__(kT) k_emit(fl_mesh_dev m, fl_domain_dev dom, i
                                              uint32_t* __restrict__ osrc, uint8_t* __restrict__ okind,
                                              const float* __restrict__ fin, float* __restrict__ fout, uint32_t C,
                                              int rule) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     __shared__ uint32_t stage[kT / 32][256];  // one column of a warp's (at most 256) new cells
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();

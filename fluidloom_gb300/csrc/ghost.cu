@@ -97,8 +97,8 @@ __global__ void __launch_bounds__(256) k_interp(fl_mesh_dev m, fl_domain_dev dom
                                                 uint32_t C, const int32_t* __restrict__ fx, const int32_t* __restrict__ fy,
                                                 const int32_t* __restrict__ fz, const uint8_t* __restrict__ flevel,
                                                 size_t nq, float* __restrict__ out) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3[12 * 512];
     fl_keys_fill_tables(t1, t3, false);
     __syncthreads();
     size_t stride = (size_t)gridDim.x * blockDim.x;

@@ -134,8 +134,8 @@ __global__ void k_deepest(const uint8_t* __restrict__ level, size_t n, uint32_t*
 // id above bit 3 * (depth - cut)); ids[i] = i.
 __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev dom, int cut,
                                                   uint64_t* __restrict__ keys, uint32_t* __restrict__ ids) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();
     const int dc = dom.depth - cut;
@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(kNbrThreads, kNbrBlocksPerSM) k_neighbours_sor
                                                                         fl_locator L, uint32_t* __restrict__ nbr,
                                                                         uint32_t* __restrict__ marks) {
     constexpr int kCells = kNbrCells / S;
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();
     const fl_probe P = fl_probe_make(t1, t3c, L, dom);

@@ -2,8 +2,7 @@
 //
 // The 12-state table is the reference's (src/core/hilbert/HilbertCodec.cpp:13-42,
 // entry = next_state << 3 | output); bit-exact keys need its values.  On the
-// GPU the table is expanded once per CTA into a 3-levels-at-a-time table in
-// shared memory (12 states x 512 inputs, entry = next_state << 9 | 9 output
+// GPU each CTA copies a 3-levels-at-a-time table into shared memory (12 states x 512 inputs, entry = next_state << 9 | 9 output
 // bits), so a 21-level key takes 7 dependent lookups instead of 21.
 #include "common.cuh"
 #include "keys.cuh"
@@ -19,8 +18,8 @@ __global__ void __launch_bounds__(kThreads) k_hilbert_encode(const int32_t* __re
                                                              const int32_t* __restrict__ z, int level,
                                                              uint64_t* __restrict__ keys,
                                                              uint32_t* __restrict__ ids, size_t n) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -35,8 +34,8 @@ __global__ void __launch_bounds__(kThreads) k_hilbert_encode(const int32_t* __re
 __global__ void __launch_bounds__(kThreads) k_hilbert_decode(const uint64_t* __restrict__ keys, int level,
                                                              int32_t* __restrict__ x, int32_t* __restrict__ y,
                                                              int32_t* __restrict__ z, size_t n) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3[12 * 512];
     fl_keys_fill_tables(t1, t3, true);
     __syncthreads();
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -86,8 +85,8 @@ __global__ void __launch_bounds__(kThreads) k_cell_keys(const int32_t* __restric
                                                         const uint8_t* __restrict__ level,
                                                         const uint16_t* __restrict__ cs, int depth, int anchor_level,
                                                         uint64_t* __restrict__ keys, size_t n) {
-    __shared__ uint8_t t1[96];
-    __shared__ uint16_t t3c[12 * 512];
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();
     size_t stride = (size_t)gridDim.x * blockDim.x;

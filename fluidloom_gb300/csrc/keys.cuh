@@ -4,7 +4,7 @@
 #pragma once
 #include "common.cuh"
 
-static __constant__ uint8_t c_enc[12][8] = {
+constexpr uint8_t kHilbertEnc[12][8] = {
     {8, 17, 27, 18, 47, 38, 28, 37},   {16, 71, 1, 62, 51, 52, 2, 61},
     {0, 75, 95, 76, 9, 10, 86, 85},    {4, 77, 55, 78, 3, 66, 80, 65},
     {50, 49, 45, 46, 67, 88, 68, 7},   {6, 57, 39, 72, 5, 58, 84, 83},
@@ -12,7 +12,7 @@ static __constant__ uint8_t c_enc[12][8] = {
     {14, 13, 81, 82, 63, 36, 24, 35},  {20, 31, 19, 56, 53, 54, 42, 41},
     {26, 93, 43, 44, 25, 94, 64, 23},  {22, 87, 21, 60, 33, 48, 34, 59},
 };
-static __constant__ uint8_t c_dec[12][8] = {
+constexpr uint8_t kHilbertDec[12][8] = {
     {8, 17, 19, 26, 30, 39, 37, 44},   {16, 2, 6, 52, 53, 63, 59, 65},
     {0, 12, 13, 73, 75, 87, 86, 90},   {86, 71, 69, 4, 0, 73, 75, 50},
     {93, 49, 48, 68, 70, 42, 43, 7},   {75, 57, 61, 87, 86, 4, 0, 34},
@@ -21,45 +21,52 @@ static __constant__ uint8_t c_dec[12][8] = {
     {70, 28, 24, 42, 43, 89, 93, 23},  {53, 36, 38, 63, 59, 18, 16, 81},
 };
 
+// The tables the key kernels keep in shared memory, worked out by the compiler: t1[s*8+q] (one
+// level) and t3[s*512+w] where w holds three levels of input (MSB level first): interleaved, 3 bits
+// a level (kCat false), or as concatenated coordinate bits x3 << 6 | y3 << 3 | z3 (kCat true), so an
+// encoder reads each 9-bit step straight from the coordinates.
+struct alignas(16) fl_key_tables {
+    uint16_t t3[12 * 512];
+    uint8_t t1[96];
+};
 
-// Fill the shared tables: t1[s*8+q] (single level) and t3[s*512+w] where w
-// packs three levels of input (MSB level first, 3 bits each).
-// Both fills are called by every thread of the block at kernel start: the
-// one-level table goes to shared memory first (scattered reads of constant
-// memory serialise across a warp), then the three-level table is built from it.
-static __device__ __forceinline__ void fl_keys_fill_tables(uint8_t* t1, uint16_t* t3, bool decode) {
-    for (int i = threadIdx.x; i < 96; i += blockDim.x) t1[i] = decode ? c_dec[i >> 3][i & 7] : c_enc[i >> 3][i & 7];
-    __syncthreads();
-    for (int i = threadIdx.x; i < 12 * 512; i += blockDim.x) {
-        unsigned s = i >> 9, w = i & 511, out = 0;
+constexpr fl_key_tables fl_make_key_tables(const uint8_t (&step)[12][8], bool cat) {
+    fl_key_tables T{};
+    for (int i = 0; i < 96; ++i) T.t1[i] = step[i >> 3][i & 7];
+    for (int i = 0; i < 12 * 512; ++i) {
+        unsigned s = (unsigned)i >> 9, out = 0;
         for (int k = 2; k >= 0; --k) {
-            unsigned q = (w >> (3 * k)) & 7u;
-            unsigned v = t1[s * 8 + q];
+            const unsigned q = cat ? ((((unsigned)i >> k) & 1u) << 2) | ((((unsigned)i >> (3 + k)) & 1u) << 1) |
+                                         (((unsigned)i >> (6 + k)) & 1u)
+                                   : ((unsigned)i >> (3 * k)) & 7u;
+            const unsigned v = step[s][q];
             out = (out << 3) | (v & 7u);
             s = v >> 3;
         }
-        t3[i] = (uint16_t)((s << 9) | out);
+        T.t3[i] = (uint16_t)((s << 9) | out);
     }
+    return T;
 }
 
-// The three-level encode table re-indexed by concatenated coordinate bits:
-// t3c[s*512 + (x3 << 6 | y3 << 3 | z3)] holds what t3 holds for the interleaved
-// input of the same three levels, so an encoder reads each 9-bit step straight
-// from the coordinates without interleaving them first.
+static __device__ const fl_key_tables g_enc_tables = fl_make_key_tables(kHilbertEnc, false);
+static __device__ const fl_key_tables g_dec_tables = fl_make_key_tables(kHilbertDec, false);
+static __device__ const fl_key_tables g_enc_tables_cat = fl_make_key_tables(kHilbertEnc, true);
+
+// Fill a block's shared tables (every thread of the block, a __syncthreads before their use; t1 and
+// t3 16-byte aligned): 774 16-byte copies from L2.  Working the three-level table out in each block
+// instead, three dependent lookups an entry, put 2 us before every key kernel's first cell (67,000 leaves:
+// k_run_keys 5.1 -> 2.9 us, k_cell_keys 5.2 -> 3.0, neighbour passes 18.6 + 13.7 -> 14.5 + 9.7).
+static __device__ __forceinline__ void fl_keys_copy_tables(const fl_key_tables& g, uint8_t* t1, uint16_t* t3) {
+    const uint4* src3 = reinterpret_cast<const uint4*>(g.t3);
+    const uint4* src1 = reinterpret_cast<const uint4*>(g.t1);
+    for (int i = threadIdx.x; i < 768; i += blockDim.x) reinterpret_cast<uint4*>(t3)[i] = __ldg(src3 + i);
+    for (int i = threadIdx.x; i < 6; i += blockDim.x) reinterpret_cast<uint4*>(t1)[i] = __ldg(src1 + i);
+}
+static __device__ __forceinline__ void fl_keys_fill_tables(uint8_t* t1, uint16_t* t3, bool decode) {
+    fl_keys_copy_tables(decode ? g_dec_tables : g_enc_tables, t1, t3);
+}
 static __device__ __forceinline__ void fl_keys_fill_tables_cat(uint8_t* t1, uint16_t* t3c) {
-    for (int i = threadIdx.x; i < 96; i += blockDim.x) t1[i] = c_enc[i >> 3][i & 7];
-    __syncthreads();
-    for (int i = threadIdx.x; i < 12 * 512; i += blockDim.x) {
-        unsigned s = i >> 9, out = 0;
-        const unsigned x3 = (i >> 6) & 7u, y3 = (i >> 3) & 7u, z3 = i & 7u;
-        for (int k = 2; k >= 0; --k) {
-            unsigned q = (((z3 >> k) & 1u) << 2) | (((y3 >> k) & 1u) << 1) | ((x3 >> k) & 1u);
-            unsigned v = t1[s * 8 + q];
-            out = (out << 3) | (v & 7u);
-            s = v >> 3;
-        }
-        t3c[i] = (uint16_t)((s << 9) | out);
-    }
+    fl_keys_copy_tables(g_enc_tables_cat, t1, t3c);
 }
 
 // hilbert::encode of the low `level` bits of x, y, z with the re-indexed table
