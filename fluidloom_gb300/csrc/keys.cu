@@ -2,8 +2,9 @@
 //
 // The 12-state table is the reference's (src/core/hilbert/HilbertCodec.cpp:13-42,
 // entry = next_state << 3 | output); bit-exact keys need its values.  On the
-// GPU each CTA copies a 3-levels-at-a-time table into shared memory (12 states x 512 inputs, entry = next_state << 9 | 9 output
-// bits), so a 21-level key takes 7 dependent lookups instead of 21.
+// GPU each CTA copies a 3-levels-at-a-time table into shared memory (12 states
+// x 512 inputs, entry = next_state << 9 | 9 output bits), so a 21-level key
+// takes 7 dependent lookups instead of 21.
 #include "common.cuh"
 #include "keys.cuh"
 
