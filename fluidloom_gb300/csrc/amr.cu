@@ -33,6 +33,7 @@
 #include "keys.cuh"
 #include "scan.cuh"
 
+#include <cstring>
 #include <vector>
 
 namespace {
@@ -775,8 +776,8 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
         FL_CHECK_LAUNCH(ctx, "k_detect");
         k_mark<<<nb, kT, 0, ctx->stream>>>(md, flags, viol, max_level, nxt, counters + 1);
         FL_CHECK_LAUNCH(ctx, "k_mark");
-        FL_TRY_CUDA(ctx, cudaMemcpyAsync(h, counters, 8, cudaMemcpyDeviceToHost, ctx->stream), "balance read");
-        FL_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "balance sync");
+        const int rc = fl_read_back(ctx, h, counters, 8, "balance read");
+        if (rc) return rc;
         r.total_violations_detected += h[0];
         if (h[0] == 0) { r.converged = 1; r.iterations = it + 1; break; }
         // k_mark ran after detection regardless; with zero violations it marks nothing
@@ -885,9 +886,11 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
     rc = fl_scan_u32_with(ctx, w.cnt, w.cnt, n, w.counters + 3, w.scan_scratch);
     if (rc) return rc;
     uint32_t hc[6] = {0, 0, 0, 0, 0, 0};
-    FL_TRY_CUDA(ctx, cudaMemcpyAsync(hc, w.counters, 24, cudaMemcpyDeviceToHost, ctx->stream), "adapt counts");
+    rc = fl_read_enqueue(ctx, 0, w.counters, sizeof(hc), "adapt counts");
+    if (rc) return rc;
     rc = fl_collect_device_status(ctx, "fl_adapt");
     if (rc) return rc;
+    std::memcpy(hc, ctx->host_read, sizeof(hc));
     s.num_groups = hc[2];
     s.num_merged = hc[2] * 8;
     s.num_split = hc[4];

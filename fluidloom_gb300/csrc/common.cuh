@@ -24,6 +24,8 @@ struct fl_ctx {
     size_t scratch_bytes = 0;
     uint32_t* dev_status = nullptr;     // device-side status words (see FL_DEVSTAT_*)
     uint32_t* host_status = nullptr;    // pinned mirror
+    char* host_read = nullptr;          // pinned landing area of small reads (kHostReadBytes)
+    cudaMemPool_t pool = nullptr;       // stream-ordered allocations (fl_dev_malloc_async)
     std::string last_error;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // fl_ctx_timer_start / stop
     void* soa = nullptr;                       // structure-of-arrays field manager (fields.cu)
@@ -39,6 +41,14 @@ struct fl_ctx {
 // allocated and cudaErrorMemoryAllocation is returned as CUDA would.
 cudaError_t fl_dev_malloc(fl_ctx* ctx, void** p, size_t bytes);
 cudaError_t fl_dev_malloc_async(fl_ctx* ctx, void** p, size_t bytes, cudaStream_t st);
+
+// Small results read back through pinned memory: enqueue the copies (at most kHostReadBytes in
+// all, `at` their place in the landing area), then wait for the stream once.  A copy into pageable
+// memory waits for the stream by itself, staged through a buffer of the driver's.
+constexpr size_t kHostReadBytes = 32768;
+int fl_read_enqueue(fl_ctx* ctx, size_t at, const void* src, size_t bytes, const char* what);
+// One such read, waited for.
+int fl_read_back(fl_ctx* ctx, void* dst, const void* src, size_t bytes, const char* what);
 
 void fl_soa_release_all(fl_ctx* ctx);
 int fl_soa_bind_external(fl_ctx* ctx, const fl_field_desc* d, size_t num_cells, size_t pitch, void* base,

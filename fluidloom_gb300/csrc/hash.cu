@@ -283,8 +283,8 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
     if (level_bound < 0) {
         k_deepest<<<fl_blocks(n, 256, ctx->num_sms * 4), 256, 0, ctx->stream>>>(m.level, n, flag);
         FL_CHECK_LAUNCH(ctx, "k_deepest");
-        FL_TRY_CUDA(ctx, cudaMemcpyAsync(hf, flag, 8, cudaMemcpyDeviceToHost, ctx->stream), "locator");
-        FL_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "locator");
+        const int rc = fl_read_back(ctx, hf, flag, 8, "locator");
+        if (rc) return rc;
     }
     L->cut = dom.anchor_level > (int)hf[1] ? dom.anchor_level - (int)hf[1] : 0;
     k_run_keys<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, dom, L->cut, keys, ids);
@@ -293,8 +293,8 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
     if (!in_key_order) {
         k_check_sorted<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(keys, n, flag);
         FL_CHECK_LAUNCH(ctx, "k_check_sorted");
-        FL_TRY_CUDA(ctx, cudaMemcpyAsync(hf, flag, 4, cudaMemcpyDeviceToHost, ctx->stream), "locator");
-        FL_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "locator");
+        const int rc = fl_read_back(ctx, hf, flag, 4, "locator");
+        if (rc) return rc;
     }
     if (hf[0]) {  // stable: equal run starts keep mesh order, so the last of them is found
         // the keys hold 3 (depth - cut) bits, plus 16 for case ids

@@ -1876,10 +1876,14 @@ int pool_topology_build(fl_ctx* ctx, fl_pool* P) {
     if (rc) return rc;
     TopoCounters h{};
     P->case_begin.assign(ncases + 1, 0);
-    FL_TRY_CUDA(ctx, cudaMemcpyAsync(&h, tc, sizeof(TopoCounters), cudaMemcpyDeviceToHost, ctx->stream), "counts");
-    FL_TRY_CUDA(ctx, cudaMemcpyAsync(P->case_begin.data(), P->d_case_begin, (ncases + 1) * 4, cudaMemcpyDeviceToHost,
-                                     ctx->stream), "case ranges");
+    static_assert(sizeof(TopoCounters) <= 1024 && 1024 + (kMaxCases + 1) * 4 <= kHostReadBytes, "pinned landing area");
+    rc = fl_read_enqueue(ctx, 0, tc, sizeof(TopoCounters), "counts");
+    if (rc) return rc;
+    rc = fl_read_enqueue(ctx, 1024, P->d_case_begin, (ncases + 1) * 4, "case ranges");
+    if (rc) return rc;
     FL_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "topology sync");
+    std::memcpy(&h, ctx->host_read, sizeof(TopoCounters));
+    std::memcpy(P->case_begin.data(), ctx->host_read + 1024, (ncases + 1) * 4);
     if (h.err & 1u) return fl_set_error(ctx, FL_E_INVALID_ARG, "brick level above the pool maximum");
     if (h.err & 6u) return fl_set_error(ctx, FL_E_INVALID_ARG, "pool bricks not in case order");
     P->lvl_off.assign(P->maxL + 2, 0);
@@ -1934,8 +1938,8 @@ int pool_topology_build(fl_ctx* ctx, fl_pool* P) {
     k_topo_sums<<<fl_blocks(n, 256, ctx->num_sms * 4), 256, 0, ctx->stream>>>(
         n, P->mesh.level, P->bclass, P->fluid, P->slow_cnt, P->slow_off, gt, P->maxL, tc);
     FL_CHECK_LAUNCH(ctx, "k_topo_sums");
-    FL_TRY_CUDA(ctx, cudaMemcpyAsync(&h, tc, sizeof(TopoCounters), cudaMemcpyDeviceToHost, ctx->stream), "sums");
-    FL_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "topology sync");
+    rc = fl_read_back(ctx, &h, tc, sizeof(TopoCounters), "sums");
+    if (rc) return rc;
     if (h.desc64 >= (1ull << 32)) return fl_set_error(ctx, FL_E_CAPACITY, "more than 2^32 stencil descriptors");
     P->num_desc = h.desc64;
     P->lvl_desc.assign(h.lvl_desc, h.lvl_desc + P->maxL + 2);

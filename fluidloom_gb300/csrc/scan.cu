@@ -15,6 +15,7 @@
 
 #include <cuda.h>
 
+#include <cstring>
 #include <mutex>
 
 namespace {
@@ -358,9 +359,11 @@ int fl_compact_and_permute(fl_ctx* ctx, const uint64_t* keys, const uint32_t* st
                                                                   ticket, total, ctx->dev_status);
     FL_CHECK_LAUNCH(ctx, "k_compact_keep");
     uint32_t m = 0;
-    FL_TRY_CUDA(ctx, cudaMemcpyAsync(&m, total, 4, cudaMemcpyDeviceToHost, ctx->stream), "total read");
+    rc = fl_read_enqueue(ctx, 0, total, 4, "total read");
+    if (rc) return rc;
     rc = fl_collect_device_status(ctx, "fl_compact_and_permute scan");
     if (rc) return rc;
+    std::memcpy(&m, ctx->host_read, 4);
     rc = fl_sort_pairs_u64_u32(ctx, sorted_keys, sorted_ids, m, 0, 64);
     if (rc) return rc;
     if (m) {
