@@ -33,6 +33,7 @@
 #include "keys.cuh"
 #include "scan.cuh"
 
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -1006,14 +1007,20 @@ int fl_neighbour_rebuild(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config
         return fl_set_error(ctx, FL_E_INVALID_ARG, "key geometry: need anchor_level <= key_depth <= 21, max level <= anchor_level, ext << anchor_level <= 2^key_depth");
     size_t n = mesh->num_cells;
     if (n == 0) return FL_OK;
-    int rc = fl_scratch_reserve(ctx, 256 + fl_align256(n * 4) + fl_locator_scratch_bytes(n));
+    int rc = fl_scratch_reserve(ctx, 256 + std::max(fl_align256(n * 4) + fl_locator_scratch_bytes(n),
+                                                    fl_neighbours_octree_scratch(n)));
     if (rc) return rc;
     Carver cv{(char*)ctx->scratch};
     void* dcase = cv.take<char>(256);
-    uint32_t* marks = cv.take<uint32_t>(n);
     fl_domain_dev dom = fl_domain_from_config(ctx, cfg, dcase);
     dom.max_level = cfg->max_refinement_level;
     fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material, mesh->case_id, n};
+    const int32_t ext[3] = {std::max(cfg->ext[0], 1), std::max(cfg->ext[1], 1), std::max(cfg->ext[2], 1)};
+    bool done = false;
+    rc = fl_neighbours_octree(ctx, md, dom, ext, subslots, cv.p, nbr, &done);
+    if (rc) return rc;
+    if (done) return fl_collect_device_status(ctx, "fl_neighbour_rebuild");
+    uint32_t* marks = cv.take<uint32_t>(n);
     fl_locator L;
     rc = fl_locator_build(ctx, md, dom, cv.p, &L);
     if (rc) return rc;

@@ -1,5 +1,5 @@
-// hash.cu — GPU open-addressing hash table (key -> index) and the neighbour
-// table rebuild built on it.
+// hash.cu — GPU open-addressing hash table (key -> index), the sorted point
+// locator and the neighbour table rebuilds.
 //
 // Replaces HashTableManager::rebuild/query (src/core/hashmap/HashTableManager.cpp:101-159,
 // which launch nothing) with the kernels they name (kernels/hashmap/hash_build.cl:19-82,
@@ -119,14 +119,37 @@ __global__ void k_hash_query(const uint64_t* __restrict__ tk, const uint32_t* __
         out[i] = fl_hash_lookup(tk, tv, lg, q[i]);
 }
 
-// flags[1] = the deepest leaf level.
-__global__ void k_deepest(const uint8_t* __restrict__ level, size_t n, uint32_t* __restrict__ flags) {
-    int deepest = 0;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        deepest = max(deepest, (int)level[i]);
-    deepest = __reduce_max_sync(0xFFFFFFFFu, deepest);
-    if ((threadIdx.x & 31) == 0 && deepest > 0) atomicMax(flags + 1, (uint32_t)deepest);
+// flags[1] = the deepest leaf level (flags[1] starts at 0), and, when `lowest` is given, *lowest = the
+// shallowest (it starts at 255).  16 levels a load, scalar loads before the first and after the last
+// 16-byte boundary: a byte per thread took 55 us for 25 M leaves, these 13.
+__global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__ level, size_t n,
+                                                     uint32_t* __restrict__ flags, uint32_t* __restrict__ lowest) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    const size_t head = min(n, (size_t)((16 - ((uintptr_t)level & 15)) & 15)), nv = (n - head) / 16;
+    const uint4* v = (const uint4*)(level + head);
+    unsigned hi4 = 0u, lo4 = 0xFFFFFFFFu;
+    for (size_t i = t; i < nv; i += stride) {
+        const uint4 w = __ldg(v + i);
+        hi4 = __vmaxu4(__vmaxu4(hi4, __vmaxu4(w.x, w.y)), __vmaxu4(w.z, w.w));
+        lo4 = __vminu4(__vminu4(lo4, __vminu4(w.x, w.y)), __vminu4(w.z, w.w));
+    }
+    unsigned hi = 0u, lo = 255u;
+    for (int k = 0; k < 32; k += 8) {
+        hi = max(hi, (hi4 >> k) & 255u);
+        lo = min(lo, (lo4 >> k) & 255u);
+    }
+    const size_t rest = n - 16 * nv;  // scalar levels: the head, then the tail
+    for (size_t i = t; i < rest; i += stride) {
+        const unsigned l = level[i < head ? i : i + 16 * nv];
+        hi = max(hi, l);
+        lo = min(lo, l);
+    }
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    if ((threadIdx.x & 31) == 0) {
+        if (hi > 0) atomicMax(flags + 1, hi);
+        if (lowest && lo < 255u) atomicMin(lowest, lo);
+    }
 }
 
 // Run start of every leaf divided by 8^cut: the anchor shifted down by cut,
@@ -252,6 +275,317 @@ __global__ void __launch_bounds__(kNbrThreads, kNbrBlocksPerSM) k_neighbours_sor
     }
 }
 
+// Octree of a single-case mesh for point location by coordinates: a dense grid of the cells of
+// level g over the domain and, below it, nodes of eight entries (child x + 2 y + 4 z).  An entry is
+// a leaf (its cell index), a node (kNodeBit | node) or kNoLeaf.  A point is found by one grid load
+// and a load per level below g, where a Hilbert key is four dependent table steps before its search
+// starts.
+constexpr uint32_t kNodeBit = 0x80000000u, kNoLeaf = 0xFFFFFFFFu;
+
+struct Octree {
+    uint32_t* grid;
+    uint32_t* node;
+    int4* node_at;    // per node its cell (x, y, z) and level
+    uint32_t* list;   // the leaves of level g and above, in any order; nullptr: all of them
+    uint32_t* state;  // [0] not usable: overlapping or outside leaves, or a gap at a node's corner;
+                      // [1] nodes, [2] leaves in list, [3] leaves with an entry below the grid
+    uint32_t node_cap;
+    int g, D;         // the grid's and the deepest level
+    int32_t dim[3];   // cells of level 0 per axis
+};
+
+__device__ __forceinline__ bool is_node(uint32_t e) { return (int32_t)e < -1; }
+
+__device__ __forceinline__ uint32_t* grid_cell(const Octree& T, int32_t x, int32_t y, int32_t z) {
+    return T.grid + ((size_t)z * (size_t)(T.dim[1] << T.g) + (size_t)y) * (size_t)(T.dim[0] << T.g) + (size_t)x;
+}
+
+__device__ __forceinline__ uint32_t* node_entry(const Octree& T, uint32_t e, int32_t x, int32_t y, int32_t z, int sh) {
+    return T.node + (size_t)(e & ~kNodeBit) * 8 + (((z >> sh) & 1) * 4 + ((y >> sh) & 1) * 2 + ((x >> sh) & 1));
+}
+
+__device__ __forceinline__ bool in_domain(const Octree& T, int32_t x, int32_t y, int32_t z, int l) {
+    return x >= 0 && y >= 0 && z >= 0 && x < (T.dim[0] << l) && y < (T.dim[1] << l) && z < (T.dim[2] << l);
+}
+
+// Exclusive prefix of v over the block in thread order (256 threads), the block's total added to
+// *counter: the block's share starts at the returned base.  One atomic per block: a same-address
+// atomic per warp alone took 0.3 ms for 20 M leaves.
+__device__ __forceinline__ uint32_t block_claim(uint32_t v, uint32_t* counter) {
+    __shared__ uint32_t s_sum[8], s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    __syncthreads();  // the last call's sums and base are read
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t run = 0;
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t t = s_sum[w];
+            s_sum[w] = run;
+            run += t;
+        }
+        s_base = run ? atomicAdd(counter, run) : 0u;
+    }
+    __syncthreads();
+    return s_base + s_sum[warp] + incl - v;
+}
+
+// The nodes, not linked yet: the leaf at a node's lowest corner makes it, with every node of its
+// chain that has the same corner (one maker per node in a mesh that fills its domain).  Four leaves
+// a thread, their loads in flight together, 1,024 consecutive leaves a block.
+constexpr int kLeafBatch = 4;
+__global__ void __launch_bounds__(256) k_octree_nodes(fl_mesh_dev m, Octree T) {
+    for (size_t i0 = (size_t)blockIdx.x * 256 * kLeafBatch; i0 < m.n; i0 += (size_t)gridDim.x * 256 * kLeafBatch) {
+        int l[kLeafBatch], make[kLeafBatch];
+        int32_t x[kLeafBatch], y[kLeafBatch], z[kLeafBatch];
+#pragma unroll
+        for (int u = 0; u < kLeafBatch; ++u) {
+            const size_t i = i0 + u * 256 + threadIdx.x;
+            l[u] = i < m.n ? m.level[i] : 0;
+            x[u] = i < m.n ? m.x[i] : 0;
+            y[u] = i < m.n ? m.y[i] : 0;
+            z[u] = i < m.n ? m.z[i] : 0;
+        }
+        uint32_t mine = 0;
+#pragma unroll
+        for (int u = 0; u < kLeafBatch; ++u) {
+            const int32_t low = x[u] | y[u] | z[u];
+            const int chain = low ? __ffs(low) - 1 : 31;  // levels up with the same lowest corner
+            make[u] = l[u] > T.g && in_domain(T, x[u], y[u], z[u], l[u]) ? min(chain, l[u] - T.g) : 0;
+            mine += (uint32_t)make[u];
+        }
+        uint32_t id = block_claim(mine, T.state + 1);
+#pragma unroll
+        for (int u = 0; u < kLeafBatch; ++u)
+            for (int k = 1; k <= make[u]; ++k, ++id) {
+                if (id < T.node_cap) T.node_at[id] = make_int4(x[u] >> k, y[u] >> k, z[u] >> k, l[u] - k);
+                else T.state[0] = 1u;
+            }
+    }
+}
+
+// The nodes of level a into their entries, those of the levels between g and a in place.
+__global__ void __launch_bounds__(256) k_octree_link(Octree T, int a) {
+    const uint32_t n = min(T.state[1], T.node_cap), stride = gridDim.x * blockDim.x;
+    for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += stride) {
+        const int4 c = T.node_at[id];
+        if (c.w != a) continue;
+        uint32_t* e = grid_cell(T, c.x >> (a - T.g), c.y >> (a - T.g), c.z >> (a - T.g));
+        for (int sh = a - T.g - 1; e && sh >= 0; --sh) {
+            const uint32_t v = *e;
+            e = is_node(v) ? node_entry(T, v, c.x, c.y, c.z, sh) : nullptr;
+        }
+        if (e) *e = kNodeBit | id;
+        else T.state[0] = 1u;
+    }
+}
+
+// The leaves: into their entry below or of the grid, or, for a leaf above the grid's level, into every
+// grid cell it covers (a warp per leaf); those of the grid's level and above also into the list,
+// unless that is every leaf (list == nullptr).  A grid cell or an entry already taken means
+// overlapping leaves; of two leaves of one cell below the grid one is lost, which the count of the
+// entries shows (k_neighbours_nodes).  The walk is a chain of L2 latencies that occupancy hides: a
+// leaf a thread at 2,048 threads an SM takes 370 us for 25 M leaves (two: 439).
+__global__ void __launch_bounds__(256, 8) k_octree_leaves(fl_mesh_dev m, Octree T) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    bool bad = false;
+    for (size_t base = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < m.n; base += stride) {
+        const size_t i = base + lane;
+        int sh = -128;  // levels below the grid; -128: nothing to place
+        int32_t x = 0, y = 0, z = 0;
+        if (i < m.n) {
+            const int l = m.level[i];
+            x = m.x[i];
+            y = m.y[i];
+            z = m.z[i];
+            if (in_domain(T, x, y, z, l)) sh = l - T.g;
+            else bad = true;
+        }
+        if (sh >= 0) {
+            uint32_t* e = grid_cell(T, x >> sh, y >> sh, z >> sh);
+            if (sh == 0) {
+                bad = bad || atomicExch(e, (uint32_t)i) != kNoLeaf;
+            } else {
+                uint32_t v = __ldcg(e);
+                for (int k = sh - 1; k >= 0 && is_node(v); --k) {
+                    e = node_entry(T, v, x, y, z, k);
+                    v = k ? __ldcg(e) : kNoLeaf - 2u;  // the leaf's own entry: below
+                }
+                const bool there = v == kNoLeaf - 2u && __ldcg(e) == kNoLeaf;
+                if (there) *e = (uint32_t)i;
+                else bad = true;
+            }
+        }
+        const bool up = sh <= 0 && sh != -128;
+        if (T.list) {
+            const unsigned all = __ballot_sync(0xFFFFFFFFu, up);
+            if (all) {
+                uint32_t first = 0;
+                if (lane == 0) first = atomicAdd(T.state + 2, (uint32_t)__popc(all));
+                first = __shfl_sync(0xFFFFFFFFu, first, 0);
+                if (up) T.list[first + (uint32_t)__popc(all & ((1u << lane) - 1u))] = (uint32_t)i;
+            }
+        }
+        for (unsigned w = __ballot_sync(0xFFFFFFFFu, up && sh < 0); w; w &= w - 1) {
+            const int j = __ffs(w) - 1;
+            const int s = -__shfl_sync(0xFFFFFFFFu, sh, j), mask = (1 << s) - 1;
+            const int32_t x0 = __shfl_sync(0xFFFFFFFFu, x, j) << s, y0 = __shfl_sync(0xFFFFFFFFu, y, j) << s,
+                          z0 = __shfl_sync(0xFFFFFFFFu, z, j) << s;
+            for (int c = lane; c < 1 << (3 * s); c += 32)
+                if (atomicExch(grid_cell(T, x0 + (c & mask), y0 + ((c >> s) & mask), z0 + (c >> (2 * s))),
+                               (uint32_t)(base + j)) != kNoLeaf)
+                    bad = true;
+        }
+    }
+    if (bad) T.state[0] = 1u;
+}
+
+// Entry r = k S + s of a row: the probe point of direction k at sub-slot s.
+struct RowProbe {
+    int dv[3], half[3];
+};
+template <int S>
+__device__ __forceinline__ RowProbe row_probe(int r) {
+    RowProbe P;
+    const int k = r / S, s = r % S, kk = k < 13 ? k : k + 1;
+    P.dv[0] = kk % 3 - 1;
+    P.dv[1] = (kk / 3) % 3 - 1;
+    P.dv[2] = kk / 9 - 1;
+    int bit = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) P.half[a] = P.dv[a] == 0 ? (s >> bit++) & 1 : 0;
+    return P;
+}
+
+// Rows of the leaves below the grid, a warp per node.  Lanes 0-26 locate the node's cell and the 26
+// of its size around it; every entry of its leaf children's rows is then the entry of one of these
+// 27 -- a leaf for all of its children, or a child of that node by one load -- so a leaf's 26
+// entries take 27 / 8 searches instead of 26, and neighbouring lanes write a row.  Latency bound (a
+// node's chain: its cell, grid, nodes, entries), so the loads of kFlight rounds of entries are in
+// flight together.  T.state[3] counts the leaves that have an entry.  25 M leaves: 869 us (1,324 us
+// with one round in flight), 1.43 ms with the octree and the rows of the grid's level, against
+// 4.51 ms for the sorted locator and its two passes of 13 searches a leaf.
+template <int S>
+__global__ void __launch_bounds__(256, 6) k_neighbours_nodes(fl_domain_dev dom, Octree T, uint32_t* __restrict__ nbr) {
+    // per row entry of the eight children: the cell the probe point lies in (0-26), its child there,
+    // for finer cells the bits of the point below the leaf's size (dv < 0: the last, else the first; a
+    // half offset at dv = 0), the leaf's child place and the entry in its row
+    constexpr int kEntries = 8 * 26 * S, kRounds = (kEntries + 31) / 32, kFlight = S == 1 ? kRounds : 9;
+    __shared__ uint32_t s_plan[kRounds * 32];
+    if (*T.state) return;  // no usable octree: the caller takes the sorted locator
+    for (int e = threadIdx.x; e < kRounds * 32; e += blockDim.x) {
+        const int c = e / (26 * S), r = e - c * (26 * S);
+        const RowProbe P = row_probe<S>(r);
+        int cell = 0, child = 0, first = 0, rest = 0, m3 = 1;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int q = ((c >> a) & 1) + P.dv[a];
+            cell += (q < 0 ? 0 : (q > 1 ? 2 : 1)) * m3;
+            child |= (q & 1) << a;
+            first |= (P.dv[a] < 0 ? 1 : P.half[a]) << a;
+            rest |= (P.dv[a] < 0 ? 1 : 0) << a;
+            m3 *= 3;
+        }
+        // past the last entry: lane 31 holds no child
+        s_plan[e] = e < kEntries ? (uint32_t)(cell | child << 5 | first << 8 | rest << 11 | c << 14 | r << 19) : 31u << 14;
+    }
+    __syncthreads();
+    const fl_domain_dev::Case d = dom.c[0];
+    const int lane = threadIdx.x & 31;
+    const int dv[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
+    const uint32_t n = T.state[1], warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t* __restrict__ node = T.node;
+    uint32_t leaves = 0;
+    for (uint32_t id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; id < n; id += warps) {
+        const int4 at = __ldg(T.node_at + id);
+        const uint32_t own = lane < 8 ? __ldg(node + ((id << 3) | lane)) : kNoLeaf;
+        const unsigned leaf8 = __ballot_sync(0xFFFFFFFFu, !is_node(own) && own != kNoLeaf);
+        if (!leaf8) continue;
+        leaves += (uint32_t)__popc(leaf8);
+        uint32_t cell = kNoLeaf;
+        if (lane < 27) {
+            int32_t p[3] = {at.x + dv[0], at.y + dv[1], at.z + dv[2]};
+            bool in = true;
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                if ((uint32_t)p[a] >= (uint32_t)(T.dim[a] << at.w)) in = in && fl_fold32(p[a], T.dim[a] << at.w, d.periodic[a]);
+            if (in) {
+                const int up = at.w - T.g;
+                cell = __ldg(grid_cell(T, p[0] >> up, p[1] >> up, p[2] >> up));
+                for (int sh = up - 1; sh >= 0 && is_node(cell); --sh)
+                    cell = __ldg(node_entry(T, cell, p[0], p[1], p[2], sh));
+            }
+        }
+#pragma unroll 1
+        for (int t0 = 0; t0 < kRounds; t0 += kFlight) {
+            uint32_t v[kFlight];
+#pragma unroll
+            for (int f = 0; f < kFlight; ++f) {  // every lane stays for the shuffles
+                const uint32_t w = t0 + f < kRounds ? s_plan[(t0 + f) * 32 + lane] : 31u << 14;
+                v[f] = __shfl_sync(0xFFFFFFFFu, cell, (int)(w & 31u));
+                if (is_node(v[f])) v[f] = __ldg(node + ((v[f] << 3) | ((w >> 5) & 7u)));  // the node bit is shifted out
+            }
+#pragma unroll
+            for (int f = 0; f < kFlight; ++f) {
+                const uint32_t w = t0 + f < kRounds ? s_plan[(t0 + f) * 32 + lane] : 31u << 14;
+                if (is_node(v[f])) {  // finer than the leaf
+                    v[f] = __ldg(node + ((v[f] << 3) | ((w >> 8) & 7u)));
+                    while (is_node(v[f])) v[f] = __ldg(node + ((v[f] << 3) | ((w >> 11) & 7u)));
+                }
+                const uint32_t i = __shfl_sync(0xFFFFFFFFu, own, (int)((w >> 14) & 31u));
+                if (!is_node(i) && i != kNoLeaf) nbr[(size_t)i * (26 * S) + (w >> 19)] = v[f];
+            }
+        }
+    }
+    if (lane == 0 && leaves) atomicAdd(T.state + 3, leaves);
+}
+
+// Rows of the leaves of the grid's level and above, a thread per entry: the probe point located from
+// the grid down.
+constexpr int kRowCells = 24;  // leaves per block at one sub-slot
+template <int S>
+__global__ void __launch_bounds__(kRowCells * 26) k_neighbours_grid(fl_mesh_dev m, fl_domain_dev dom, Octree T,
+                                                                    uint32_t* __restrict__ nbr) {
+    if (*T.state) return;
+    constexpr int kCells = kRowCells / S;
+    const int cl = threadIdx.x / (26 * S);
+    const int r = threadIdx.x - cl * (26 * S);
+    const RowProbe P = row_probe<S>(r);
+    const fl_domain_dev::Case d = dom.c[0];
+    const uint32_t n = T.list ? T.state[2] : (uint32_t)m.n;
+    for (uint32_t base = blockIdx.x * kCells; base < n; base += gridDim.x * kCells) {
+        const uint32_t j = base + cl;
+        if (j >= n) continue;
+        const uint32_t i = T.list ? __ldg(T.list + j) : j;
+        const int sh = T.D - m.level[i];
+        const int32_t size = 1 << sh, mid = size >> 1;
+        int32_t p[3] = {m.x[i] << sh, m.y[i] << sh, m.z[i] << sh};
+        bool in = true;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            p[a] += P.dv[a] < 0 ? -1 : (P.dv[a] > 0 ? size : (P.half[a] ? mid : 0));
+            if ((uint32_t)p[a] >= (uint32_t)(T.dim[a] << T.D)) in = in && fl_fold32(p[a], T.dim[a] << T.D, d.periodic[a]);
+        }
+        uint32_t e = kNoLeaf;
+        if (in) {
+            int b = T.D - T.g;
+            e = __ldg(grid_cell(T, p[0] >> b, p[1] >> b, p[2] >> b));
+            while (is_node(e)) {
+                --b;
+                e = __ldg(node_entry(T, e, p[0], p[1], p[2], b));
+            }
+        }
+        nbr[(size_t)i * (26 * S) + r] = e;
+    }
+}
+
 int locator_log2nb(size_t n) {
     int lg = 0;
     while ((1ull << lg) < n) ++lg;
@@ -281,8 +615,8 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
     FL_TRY_CUDA(ctx, cudaMemsetAsync(flag, 0, 8, ctx->stream), "locator");
     uint32_t hf[2] = {0, (uint32_t)std::max(level_bound, 0)};  // unsorted, deepest level
     if (level_bound < 0) {
-        k_deepest<<<fl_blocks(n, 256, ctx->num_sms * 4), 256, 0, ctx->stream>>>(m.level, n, flag);
-        FL_CHECK_LAUNCH(ctx, "k_deepest");
+        k_level_range<<<fl_blocks((n + 15) / 16, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m.level, n, flag, nullptr);
+        FL_CHECK_LAUNCH(ctx, "k_level_range");
         const int rc = fl_read_back(ctx, hf, flag, 8, "locator");
         if (rc) return rc;
     }
@@ -326,6 +660,83 @@ int fl_neighbours_sorted(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev&
     }
     FL_CHECK_LAUNCH(ctx, "k_neighbours_sorted");
     return FL_OK;
+}
+
+// The octree's grid has at most two cells per leaf: its level g is the deepest that fits, at most
+// kGridFill levels below the shallowest leaf (a leaf above the grid fills 8^(g - level) cells).
+constexpr int kGridFill = 4;
+constexpr int kMostNodeLevels = 8;  // below the grid: a pass over the nodes and a load per search each
+
+static size_t octree_most_cells(size_t n) { return std::max<size_t>(2 * n, 64); }
+
+size_t fl_neighbours_octree_scratch(size_t n) {
+    return 256 + fl_align256(octree_most_cells(n) * 4) + fl_align256((n / 7 + 1) * 32) + fl_align256((n / 7 + 1) * 16) +
+           fl_align256(n * 4);
+}
+
+int fl_neighbours_octree(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom, const int32_t* ext, int subslots,
+                         void* scratch, uint32_t* nbr, bool* done) {
+    *done = false;
+    const size_t n = m.n, most = octree_most_cells(n);
+    if (m.case_id || n >= kNodeBit) return FL_OK;  // so nodes * 8 stays below 2^32
+    Octree T{};
+    char* p = (char*)scratch;
+    T.node_cap = (uint32_t)(n / 7 + 1);
+    T.state = (uint32_t*)p; p += 256;
+    T.grid = (uint32_t*)p; p += fl_align256(most * 4);
+    T.node = (uint32_t*)p; p += fl_align256((size_t)T.node_cap * 32);
+    T.node_at = (int4*)p; p += fl_align256((size_t)T.node_cap * 16);
+    T.list = (uint32_t*)p;
+    uint32_t* range = T.state + 8;  // [1] deepest, [2] shallowest
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(T.state, 0, 40, ctx->stream), "octree state");
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(range + 2, 0xFF, 4, ctx->stream), "octree state");
+    k_level_range<<<fl_blocks((n + 15) / 16, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m.level, n, range, range + 2);
+    FL_CHECK_LAUNCH(ctx, "k_level_range");
+    uint32_t h[3];
+    int rc = fl_read_back(ctx, h, range, 12, "level range");
+    if (rc) return rc;
+    T.D = (int)h[1];
+    const int lowest = h[2] > 254 ? 0 : (int)h[2];
+    size_t cells = 1;
+    for (int a = 0; a < 3; ++a) {
+        T.dim[a] = ext[a];
+        cells = cells > most ? cells : cells * (size_t)ext[a];
+    }
+    if (T.D > dom.anchor_level || T.D > dom.max_level || cells > most) return FL_OK;
+    while (T.g < T.D && T.g < lowest + kGridFill && cells * 8 <= most) {
+        ++T.g;
+        cells *= 8;
+    }
+    if (T.D - T.g > kMostNodeLevels) return FL_OK;
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(T.grid, 0xFF, cells * 4, ctx->stream), "octree grid");
+    const unsigned nb = fl_blocks((n + kLeafBatch - 1) / kLeafBatch, 256, ctx->num_sms * 8);
+    if (T.D > T.g) {
+        FL_TRY_CUDA(ctx, cudaMemsetAsync(T.node, 0xFF, (size_t)T.node_cap * 32, ctx->stream), "octree nodes");
+        k_octree_nodes<<<nb, 256, 0, ctx->stream>>>(m, T);
+        FL_CHECK_LAUNCH(ctx, "k_octree_nodes");
+        for (int a = T.g; a < T.D; ++a) {
+            k_octree_link<<<fl_blocks(T.node_cap, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(T, a);
+            FL_CHECK_LAUNCH(ctx, "k_octree_link");
+        }
+    }
+    if (T.D == T.g) T.list = nullptr;
+    k_octree_leaves<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, T);
+    FL_CHECK_LAUNCH(ctx, "k_octree_leaves");
+    const size_t per_block = (size_t)(kRowCells / subslots);
+    const unsigned rows = (unsigned)std::min<size_t>((n + per_block - 1) / per_block, (size_t)ctx->num_sms * 6);
+    if (subslots == 4) k_neighbours_grid<4><<<rows, kRowCells * 26, 0, ctx->stream>>>(m, dom, T, nbr);
+    else k_neighbours_grid<1><<<rows, kRowCells * 26, 0, ctx->stream>>>(m, dom, T, nbr);
+    FL_CHECK_LAUNCH(ctx, "k_neighbours_grid");
+    if (T.D > T.g) {
+        const unsigned wb = fl_blocks((size_t)T.node_cap * 32, 256, ctx->num_sms * 16);
+        if (subslots == 4) k_neighbours_nodes<4><<<wb, 256, 0, ctx->stream>>>(dom, T, nbr);
+        else k_neighbours_nodes<1><<<wb, 256, 0, ctx->stream>>>(dom, T, nbr);
+        FL_CHECK_LAUNCH(ctx, "k_neighbours_nodes");
+    }
+    uint32_t st[4];
+    rc = fl_read_back(ctx, st, T.state, sizeof(st), "octree state");
+    *done = !rc && !st[0] && (!T.list || (size_t)st[2] + st[3] == n);
+    return rc;
 }
 
 int fl_hash_lg(uint64_t cap) {
