@@ -1191,62 +1191,87 @@ struct PoolView {
     int parity[16];
     const LbmCaseDev* cases;
     const uint8_t* mnear;  // k_mask_near bits of the current mesh, or nullptr (no case has a mask)
+    const uint8_t* bclass;  // k_brick_table's classes and own-site solid words
+    const uint32_t* smask;
 };
 
 __device__ __forceinline__ const float* cur_buf(const PoolView& p, int l) { return p.parity[l] ? p.f1 : p.f0; }
 
+// The solid bits of the x-quad at site `own` of brick b, from its class: interior bricks hold no solid
+// site, all-solid bricks only solid ones, general bricks' words say (solid_at per site, with its
+// 64-bit voxel arithmetic, cost more than the populations' loads).
+__device__ __forceinline__ uint32_t solid_quad(const PoolView& p, size_t b, int own) {
+    const int k = p.bclass[b];
+    if (k == 0) return 0u;
+    return k == 2 ? 0xFu : (p.smask[b * 16 + (own >> 5)] >> (own & 31)) & 0xFu;
+}
+
 // Per-brick max |curl u| (physical scale 2^level), central differences inside
 // the brick, one-sided at its faces; 0 in solid sites (oracle: brick_vorticity).
-__global__ void __launch_bounds__(512) k_vorticity(PoolView p, size_t n, float* __restrict__ wmax,
-                                                   unsigned* __restrict__ case_max) {
-    __shared__ float U[3][512];
-    __shared__ float red[16];
+// A thread takes an x-quad, its 19 loads of 16 bytes in flight together: DRAM
+// bound, 25,065 bricks (0.98 GB read) 203 -> 170 us (a site a thread before).
+__global__ void __launch_bounds__(128, 4) k_vorticity(PoolView p, size_t n, float* __restrict__ wmax,
+                                                      unsigned* __restrict__ case_max) {
+    __shared__ __align__(16) float U[3][512];
+    __shared__ float red[4];
+    const int t = threadIdx.x;
+    const int x0 = (t & 1) * 4, y = (t >> 1) & 7, z = t >> 4;
+    const int own = x0 + 8 * y + 64 * z;
     for (size_t b = blockIdx.x; b < n; b += gridDim.x) {
-        const int s = threadIdx.x;
         const int l = p.blevel[b];
-        const LbmCaseDev& c = p.cases[p.bcase[b]];
         const float* F = cur_buf(p, l);
-        int64_t G[3] = {(int64_t)p.bx[b] * 8 + (s & 7), (int64_t)p.by[b] * 8 + ((s >> 3) & 7),
-                        (int64_t)p.bz[b] * 8 + (s >> 6)};
-        if (solid_at(c, G[0], G[1], G[2], l)) {
-            U[0][s] = U[1][s] = U[2][s] = 0.0f;
-        } else {
-            float f[Q];
+        float f[Q][4];
 #pragma unroll
-            for (int q = 0; q < Q; ++q) f[q] = F[fidx(p.cap, q, b, s)];
+        for (int q = 0; q < Q; ++q) {
+            const float4 v = __ldg((const float4*)(F + fidx(p.cap, q, b, own)));
+            f[q][0] = v.x; f[q][1] = v.y; f[q][2] = v.z; f[q][3] = v.w;
+        }
+        const uint32_t solid4 = solid_quad(p, b, own);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float g[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) g[q] = f[q][i];
             float rho, jx, jy, jz;
-            moments(f, rho, jx, jy, jz);
-            float inv = 1.0f / rho;
-            U[0][s] = jx * inv; U[1][s] = jy * inv; U[2][s] = jz * inv;
+            moments(g, rho, jx, jy, jz);
+            const float inv = 1.0f / rho;
+            const bool solid = (solid4 >> i) & 1u;
+            U[0][own + i] = solid ? 0.0f : jx * inv;
+            U[1][own + i] = solid ? 0.0f : jy * inv;
+            U[2][own + i] = solid ? 0.0f : jz * inv;
         }
         __syncthreads();
-        const int co[3] = {s & 7, (s >> 3) & 7, s >> 6};
-        auto dd = [&](int comp, int axis) {
-            int stride = axis == 0 ? 1 : (axis == 1 ? 8 : 64);
-            if (co[axis] == 0) return U[comp][s + stride] - U[comp][s];
-            if (co[axis] == 7) return U[comp][s] - U[comp][s - stride];
-            float t = U[comp][s + stride] - U[comp][s - stride];
-            return t * 0.5f;
-        };
-        float wx = dd(2, 1) - dd(1, 2);
-        float wy = dd(0, 2) - dd(2, 0);
-        float wz = dd(1, 0) - dd(0, 1);
-        float w2 = wx * wx;
-        w2 = w2 + wy * wy;
-        w2 = w2 + wz * wz;
-        float mag = sqrtf(w2) * (float)(1 << l);
-        for (int o = 16; o > 0; o >>= 1) mag = fmaxf(mag, __shfl_xor_sync(0xFFFFFFFFu, mag, o));
-        if ((s & 31) == 0) red[s >> 5] = mag;
-        __syncthreads();
-        if (s < 32) {
-            float m = s < 16 ? red[s] : 0.0f;
-            for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-            if (s == 0) {
-                wmax[b] = m;
-                atomicMax(case_max + p.bcase[b], __float_as_uint(m));  // non-negative floats order as uints
-            }
+        float most = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int s = own + i;
+            const int co[3] = {x0 + i, y, z};
+            auto dd = [&](int comp, int axis) {
+                const int stride = axis == 0 ? 1 : (axis == 1 ? 8 : 64);
+                if (co[axis] == 0) return U[comp][s + stride] - U[comp][s];
+                if (co[axis] == 7) return U[comp][s] - U[comp][s - stride];
+                float d = U[comp][s + stride] - U[comp][s - stride];
+                return d * 0.5f;
+            };
+            float wx = dd(2, 1) - dd(1, 2);
+            float wy = dd(0, 2) - dd(2, 0);
+            float wz = dd(1, 0) - dd(0, 1);
+            float w2 = wx * wx;
+            w2 = w2 + wy * wy;
+            w2 = w2 + wz * wz;
+            const float mag = sqrtf(w2) * (float)(1 << l);
+            most = i == 0 ? mag : fmaxf(most, mag);  // NaN only where every site's is, as fmaxf has it
         }
+        for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xFFFFFFFFu, most, o));
+        if ((t & 31) == 0) red[t >> 5] = most;
         __syncthreads();
+        if (t == 0) {
+            const float m = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+            wmax[b] = m;
+            atomicMax(case_max + p.bcase[b], __float_as_uint(m));  // non-negative floats order as uints
+        }
+        // U is next written after the next brick's loads: every thread has passed the barrier above
+        // and read U before it; red is read by thread 0 before it reaches the next barrier
     }
 }
 
@@ -1340,21 +1365,14 @@ __global__ void __launch_bounds__(128) k_brick_sums(PoolView p, size_t n, float*
     const int x0 = (t & 1) * 4, y = (t >> 1) & 7, z = t >> 4;
     const int own = x0 + 8 * y + 64 * z;
     for (size_t b = blockIdx.x; b < n; b += gridDim.x) {
-        const int l = p.blevel[b];
-        const LbmCaseDev& c = p.cases[p.bcase[b]];
-        const float* F = cur_buf(p, l);
+        const float* F = cur_buf(p, p.blevel[b]);
         float f[Q][4];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             const float4 v = __ldg((const float4*)(F + fidx(p.cap, q, b, own)));
             f[q][0] = v.x; f[q][1] = v.y; f[q][2] = v.z; f[q][3] = v.w;
         }
-        uint32_t solid4 = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (solid_at(c, (int64_t)p.bx[b] * 8 + x0 + i, (int64_t)p.by[b] * 8 + y, (int64_t)p.bz[b] * 8 + z, l))
-                solid4 |= 1u << i;
-        brick_sums_store(f, solid4, b, part);
+        brick_sums_store(f, solid_quad(p, b, own), b, part);
     }
 }
 
@@ -1367,9 +1385,8 @@ __global__ void __launch_bounds__(128) k_macroscopic(PoolView p, size_t n, float
     const int x0 = (t & 1) * 4, y = (t >> 1) & 7, z = t >> 4;
     const int own = x0 + 8 * y + 64 * z;
     for (size_t b = blockIdx.x; b < n; b += gridDim.x) {
-        const int l = p.blevel[b];
-        const LbmCaseDev& c = p.cases[p.bcase[b]];
-        const float* F = cur_buf(p, l);
+        const float* F = cur_buf(p, p.blevel[b]);
+        const uint32_t solid4 = solid_quad(p, b, own);
         float4 v4[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) v4[q] = __ldg((const float4*)(F + fidx(p.cap, q, b, own)));
@@ -1381,8 +1398,7 @@ __global__ void __launch_bounds__(128) k_macroscopic(PoolView p, size_t n, float
             for (int q = 0; q < Q; ++q) f[q] = i == 0 ? v4[q].x : (i == 1 ? v4[q].y : (i == 2 ? v4[q].z : v4[q].w));
             float r, jx, jy, jz;
             moments(f, r, jx, jy, jz);
-            const bool solid =
-                solid_at(c, (int64_t)p.bx[b] * 8 + x0 + i, (int64_t)p.by[b] * 8 + y, (int64_t)p.bz[b] * 8 + z, l);
+            const bool solid = (solid4 >> i) & 1u;
             const float inv = 1.0f / r;
             o[0][i] = solid ? 0.0f : r;
             o[1][i] = solid ? 0.0f : jx * inv;
@@ -1397,50 +1413,57 @@ __global__ void __launch_bounds__(128) k_macroscopic(PoolView p, size_t n, float
     }
 }
 
-// Per chunk of up to 1024 consecutive bricks of one case (one CTA each): the
-// bricks' partials summed in a fixed order -- thread t takes bricks t, t+256,
-// ..., then a fixed tree across threads.  Chunks start at each case's first
-// brick, so a case's sums do not depend on the other cases of the pool.
-constexpr uint32_t kChunkBricks = 1024;
+// Per chunk of up to kChunkBricks consecutive bricks of one case (one CTA each),
+// a thread per brick and component (component fastest, so a brick's warp
+// partials are read in 32-byte pieces): the brick's four warp totals in order,
+// then a fixed tree over the bricks.  Chunks start at each case's first brick,
+// so a case's sums do not depend on the other cases of the pool.  FP64
+// instructions issue at a small fraction of the FP32 rate, so the work is spread
+// over many small CTAs: 2,938 bricks 24.8 us in 3 chunks of 1,024, 5.5 now.
+constexpr uint32_t kChunkBricks = 128;
 
-__global__ void __launch_bounds__(256) k_chunk_sums(const float* __restrict__ part, const uint8_t* __restrict__ level,
-                                                    const uint2* __restrict__ chunks, uint32_t nchunks,
-                                                    double* __restrict__ chunk_part) {
-    __shared__ double red[4][256];
+__global__ void __launch_bounds__(4 * kChunkBricks) k_chunk_sums(const float* __restrict__ part,
+                                                                 const uint8_t* __restrict__ level,
+                                                                 const uint2* __restrict__ chunks, uint32_t nchunks,
+                                                                 double* __restrict__ chunk_part) {
+    __shared__ double red[4 * kChunkBricks];
+    const int k = threadIdx.x & 3;
     for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const uint2 r = chunks[c];
-        double acc[4] = {0, 0, 0, 0};
-        for (uint32_t b = r.x + threadIdx.x; b < r.y; b += 256) {
+        const uint32_t b = r.x + (threadIdx.x >> 2);
+        double acc = 0.0;
+        if (b < r.y) {
             // the brick's four warp totals in order, times its site volume 8^-level (exact)
             const double vol = __longlong_as_double((long long)(1023 - 3 * (int)level[b]) << 52);
-            const float* w = part + (size_t)b * 32;
-            for (int k = 0; k < 4; ++k) {
-                double s4 = (double)w[2 * k] + (double)w[2 * k + 1];
-                for (int v = 1; v < 4; ++v) s4 = s4 + ((double)w[v * 8 + 2 * k] + (double)w[v * 8 + 2 * k + 1]);
-                acc[k] += s4 * vol;
-            }
+            float2 w[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) w[v] = __ldg((const float2*)(part + (size_t)b * 32 + v * 8 + 2 * k));
+            double s4 = (double)w[0].x + (double)w[0].y;
+#pragma unroll
+            for (int v = 1; v < 4; ++v) s4 = s4 + ((double)w[v].x + (double)w[v].y);
+            acc = s4 * vol;
         }
-        for (int k = 0; k < 4; ++k) red[k][threadIdx.x] = acc[k];
+        red[threadIdx.x] = acc;
         __syncthreads();
-        for (int o = 128; o > 0; o >>= 1) {
-            if (threadIdx.x < o)
-                for (int k = 0; k < 4; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
+        for (int o = 2 * kChunkBricks; o >= 4; o >>= 1) {
+            if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
             __syncthreads();
         }
-        if (threadIdx.x < 4) chunk_part[(size_t)c * 4 + threadIdx.x] = red[threadIdx.x][0];
+        if (threadIdx.x < 4) chunk_part[(size_t)c * 4 + threadIdx.x] = red[threadIdx.x];
         __syncthreads();
     }
 }
 
-// Per case (thread = case and component): its chunks' sums in chunk order.
+// A warp per case and component: its chunks' sums, lane by lane in chunk order, then a fixed tree.
 __global__ void k_case_sums(const double* __restrict__ chunk_part, const uint32_t* __restrict__ case_chunk,
                             int ncases, double* __restrict__ out) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (t >= ncases * 4) return;
     const int cs = t >> 2, k = t & 3;
     double s = 0.0;
-    for (uint32_t c = case_chunk[cs]; c < case_chunk[cs + 1]; ++c) s += chunk_part[(size_t)c * 4 + k];
-    out[t] = s;
+    for (uint32_t c = case_chunk[cs] + lane; c < case_chunk[cs + 1]; c += 32) s += chunk_part[(size_t)c * 4 + k];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if (lane == 0) out[t] = s;
 }
 
 // exp(x) for x <= 0 from the mathematics: x = n ln2 + r with |r| <= ln2/2
@@ -1607,7 +1630,7 @@ struct fl_pool {
     std::vector<uint32_t> case_begin;
     uint32_t* d_case_begin = nullptr;
     TopoCounters* d_topo = nullptr;       // k_topo_bins / k_topo_sums results
-    uint2* d_chunks = nullptr;            // brick ranges of <= 1024 bricks, each within one case
+    uint2* d_chunks = nullptr;            // brick ranges of <= kChunkBricks bricks, each within one case
     uint32_t* d_case_chunk = nullptr;     // per case: first chunk; [ncases] = end
     double* chunk_part = nullptr;
     uint32_t nchunks = 0;
@@ -1704,6 +1727,8 @@ PoolView view(fl_pool* P) {
     for (int l = 0; l < 16; ++l) v.parity[l] = P->parity[l];
     v.cases = P->d_cases;
     v.mnear = P->any_mask ? P->mnear : nullptr;
+    v.bclass = P->bclass;
+    v.smask = P->smask;
     return v;
 }
 
@@ -1996,7 +2021,7 @@ int pool_flags(fl_ctx* ctx, fl_pool* P, int use_vorticity) {
     PoolView v = view(P);
     FL_TRY_CUDA(ctx, cudaMemsetAsync(P->case_max, 0, P->cases.size() * 4, ctx->stream), "case max");
     if (use_vorticity) {
-        k_vorticity<<<fl_blocks(n, 1, ctx->num_sms * 8), 512, 0, ctx->stream>>>(v, n, P->wmax, P->case_max);
+        k_vorticity<<<fl_blocks(n, 1, ctx->num_sms * 8), 128, 0, ctx->stream>>>(v, n, P->wmax, P->case_max);
         FL_CHECK_LAUNCH(ctx, "k_vorticity");
     }
     k_flags<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(v, n, P->wmax, P->case_max, use_vorticity,
@@ -2706,11 +2731,11 @@ int fl_pool_conservation_async(fl_ctx* ctx, fl_pool* P, double* out) {
     }
     int nc = (int)P->cases.size();
     if (P->nchunks) {
-        k_chunk_sums<<<std::min<uint32_t>(P->nchunks, (uint32_t)ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+        k_chunk_sums<<<std::min<uint32_t>(P->nchunks, (uint32_t)ctx->num_sms * 4), 4 * kChunkBricks, 0, ctx->stream>>>(
             P->part, P->mesh.level, P->d_chunks, P->nchunks, P->chunk_part);
         FL_CHECK_LAUNCH(ctx, "k_chunk_sums");
     }
-    k_case_sums<<<(nc * 4 + 255) / 256, 256, 0, ctx->stream>>>(P->chunk_part, P->d_case_chunk, nc, P->cons);
+    k_case_sums<<<(nc * 4 + 7) / 8, 256, 0, ctx->stream>>>(P->chunk_part, P->d_case_chunk, nc, P->cons);
     FL_CHECK_LAUNCH(ctx, "k_case_sums");
     FL_TRY_CUDA(ctx, cudaMemcpyAsync(out, P->cons, nc * 32, cudaMemcpyDefault, ctx->stream), "conservation");
     return FL_OK;
