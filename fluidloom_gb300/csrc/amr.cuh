@@ -16,9 +16,11 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
                    const uint32_t* tv, uint64_t cap, const fl_locator* L, int mode, int max_level, int max_iters,
                    uint8_t* shadow, uint8_t* viol, uint8_t* act, uint32_t* counters, fl_balance_result* res,
                    bool balanced_input = false);
-// level_bound >= 0: no cell of the mesh is deeper (the point locator then skips a host read).
+// level_bound >= 0: no cell of the mesh is deeper; in_key_order: its cells are in key order (the
+// point locator then skips a host read each).
 int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const fl_domain_dev& dom,
-                     bool run_balance, void* scratch, size_t* M_out, fl_adapt_stats* st, int level_bound = -1);
+                     bool run_balance, void* scratch, size_t* M_out, fl_adapt_stats* st, int level_bound = -1,
+                     bool in_key_order = false);
 int fl_adapt_finish(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const fl_domain_dev& dom,
                     void* scratch, size_t M, const float* fields, uint32_t C, fl_mesh* out, float* out_fields,
                     uint32_t* osrc, uint8_t* okind, uint32_t* omembers, uint32_t num_groups);

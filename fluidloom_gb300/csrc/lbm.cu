@@ -145,22 +145,22 @@ __device__ __forceinline__ DS ds_add(DS a, DS b) {
 // a coarser site samples the voxel at its centre (the upper of the two middle
 // ones), a finer site the voxel that holds it; sites outside the case grid are
 // fluid.
-__device__ __forceinline__ bool mask_at(const LbmCaseDev& c, int64_t sx, int64_t sy, int64_t sz, int l) {
-    const int64_t G[3] = {sx, sy, sz};
-    int64_t v[3], N[3];
+__device__ __forceinline__ bool mask_at(const LbmCaseDev& c, int32_t sx, int32_t sy, int32_t sz, int l) {
+    const int32_t G[3] = {sx, sy, sz};  // at most 16 bricks of 8 sites << 13 an axis: 2^20
+    int32_t v[3], N[3];
     const int sh = c.mask_level - l;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        if (G[a] < 0 || G[a] >= ((int64_t)c.ext[a] * 8 << l)) return false;
-        N[a] = (int64_t)c.ext[a] * 8 << c.mask_level;
-        v[a] = sh >= 0 ? (G[a] << sh) + (sh ? (int64_t)1 << (sh - 1) : 0) : G[a] >> -sh;
+        if (G[a] < 0 || G[a] >= (c.ext[a] * 8 << l)) return false;
+        N[a] = c.ext[a] * 8 << c.mask_level;
+        v[a] = sh >= 0 ? (G[a] << sh) + (sh ? 1 << (sh - 1) : 0) : G[a] >> -sh;
     }
     const uint64_t i = ((uint64_t)v[2] * (uint64_t)N[1] + (uint64_t)v[1]) * (uint64_t)N[0] + (uint64_t)v[0];
     return (__ldg(c.mask + (i >> 5)) >> (i & 31)) & 1u;
 }
 
 // A site is solid inside the case's sphere or on a voxel of its solid mask.
-__device__ __forceinline__ bool solid_at(const LbmCaseDev& c, int64_t sx, int64_t sy, int64_t sz, int l) {
+__device__ __forceinline__ bool solid_at(const LbmCaseDev& c, int32_t sx, int32_t sy, int32_t sz, int l) {
     if (c.has_sphere) {
         float inv = 1.0f / (float)(1 << l);
         float px = ((float)sx + 0.5f) * inv, py = ((float)sy + 0.5f) * inv, pz = ((float)sz + 0.5f) * inv;
@@ -383,22 +383,21 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t kind, int q, int s, uint3
 }
 
 struct BrickTopo {
-    uint32_t nbr[104];  // 26 directions x 4 sub-slots
-    uint8_t nlv[104];   // their levels (0xFF: none)
-    uint32_t nb27[27];
+    uint32_t nbr[104];    // 26 directions x 4 sub-slots
+    uint8_t nlv[104];     // their levels (0xFF: none)
+    int32_t org[104][3];  // their first sites
     uint32_t solid[32];  // 10^3 bits: the brick and its one-site halo
     int near;
 };
 
-__device__ uint64_t resolve_source(const LbmCaseDev& c, const int32_t* bx, const int32_t* by, const int32_t* bz,
-                                   uint32_t b, int q, int l, int s, const int64_t* G0, const BrickTopo& T,
-                                   uint32_t* dev_status) {
+__device__ uint64_t resolve_source(const LbmCaseDev& c, uint32_t b, int q, int l, int s, const int32_t* G0,
+                                   const BrickTopo& T, uint32_t* dev_status) {
     const uint32_t own = b * 512u + (uint32_t)s;
     const int sx = s & 7, sy = (s >> 3) & 7, sz = s >> 6;
     const int lx = sx - CXq(q), ly = sy - CYq(q), lz = sz - CZq(q);
-    int64_t S[3] = {G0[0] + lx, G0[1] + ly, G0[2] + lz};
-    int64_t N[3];
-    for (int ax = 0; ax < 3; ++ax) N[ax] = ((int64_t)c.ext[ax] * 8) << l;
+    const int32_t S[3] = {G0[0] + lx, G0[1] + ly, G0[2] + lz};
+    int32_t N[3];
+    for (int ax = 0; ax < 3; ++ax) N[ax] = (c.ext[ax] * 8) << l;
     int out_face[3] = {-1, -1, -1};
     bool out = false;
     for (int ax = 0; ax < 3; ++ax) {
@@ -419,7 +418,7 @@ __device__ uint64_t resolve_source(const LbmCaseDev& c, const int32_t* bx, const
         if (outlet) return make_desc(kSrcOutlet, q, s, own);
         return make_desc(moving ? kSrcWall : kSrcBounce, q, s, own);
     }
-    int64_t Sw[3];  // the source is one site from G: wrapping is one add or subtract
+    int32_t Sw[3];  // the source is one site from G: wrapping is one add or subtract
     for (int ax = 0; ax < 3; ++ax)
         Sw[ax] = !c.periodic[ax] ? S[ax] : (S[ax] < 0 ? S[ax] + N[ax] : (S[ax] >= N[ax] ? S[ax] - N[ax] : S[ax]));
     if (T.near && solid_bit(T.solid, lx, ly, lz)) return make_desc(kSrcBounce, q, s, own);
@@ -432,14 +431,15 @@ __device__ uint64_t resolve_source(const LbmCaseDev& c, const int32_t* bx, const
         if (d[ax] == 0) { if (L3[ax] >= 4) sub_slot |= 1 << bit; ++bit; }
     int kk = (d[2] + 1) * 9 + (d[1] + 1) * 3 + (d[0] + 1);
     int k = kk < 13 ? kk : kk - 1;
-    uint32_t nb = T.nbr[k * 4 + sub_slot];
+    const int slot = k * 4 + sub_slot;
+    uint32_t nb = T.nbr[slot];
     if (nb == FL_INVALID_INDEX) return make_desc(kSrcBounce, q, s, own);
-    int ln = T.nlv[k * 4 + sub_slot];
-    int64_t nx = (int64_t)bx[nb] * 8, ny = (int64_t)by[nb] * 8, nz = (int64_t)bz[nb] * 8;
+    int ln = T.nlv[slot];
+    const int32_t nx = T.org[slot][0], ny = T.org[slot][1], nz = T.org[slot][2];
     if (ln == l)
         return make_desc(kSrcSame, q, s, nb * 512u + (uint32_t)((Sw[0] - nx) + 8 * (Sw[1] - ny) + 64 * (Sw[2] - nz)));
     if (ln == l - 1) {
-        int64_t px = (Sw[0] >> 1) - nx, py = (Sw[1] >> 1) - ny, pz = (Sw[2] >> 1) - nz;
+        const int32_t px = (Sw[0] >> 1) - nx, py = (Sw[1] >> 1) - ny, pz = (Sw[2] >> 1) - nz;
         if (px < 0 || px > 7 || py < 0 || py > 7 || pz < 0 || pz > 7) {
             atomicAdd(dev_status + FL_DEVSTAT_BOUNDS, 1u);
             return make_desc(kSrcBounce, q, s, own);
@@ -447,7 +447,7 @@ __device__ uint64_t resolve_source(const LbmCaseDev& c, const int32_t* bx, const
         return make_desc(kSrcCoarse, q, s, nb * 512u + (uint32_t)(px + 8 * py + 64 * pz));
     }
     if (ln == l + 1) {  // children 2S .. 2S+1 per axis; 2S - n is even, so one test per axis
-        int64_t px = 2 * Sw[0] - nx, py = 2 * Sw[1] - ny, pz = 2 * Sw[2] - nz;
+        const int32_t px = 2 * Sw[0] - nx, py = 2 * Sw[1] - ny, pz = 2 * Sw[2] - nz;
         if (px < 0 || px > 6 || py < 0 || py > 6 || pz < 0 || pz > 6) {
             atomicAdd(dev_status + FL_DEVSTAT_BOUNDS, 1u);
             return make_desc(kSrcBounce, q, s, own);
@@ -461,8 +461,12 @@ __device__ uint64_t resolve_source(const LbmCaseDev& c, const int32_t* bx, const
 // The descriptors of the general bricks, from k_brick_table's tables: one
 // CTA per brick, one thread per descriptor.  Descriptor k of a brick lies in
 // the x-quad with the largest first offset <= k (qmask .w); inside the quad
-// they run q-major, then site.  Written to desc + off[p] + k.
-__global__ void __launch_bounds__(256, 4) k_slow_emit(size_t ng, const uint32_t* __restrict__ gen,
+// they run q-major, then site.  Written to desc + off[p] + k.  A brick is a chain
+// of dependent loads (its place, its neighbours, their levels and origins)
+// before its threads can start, so many small CTAs are kept in flight
+// (25,065 bricks: 256 threads at 4 per SM 134 us, 113 with 32-bit sites, these 89).
+constexpr int kEmitCtas = 12;  // per SM
+__global__ void __launch_bounds__(128, kEmitCtas) k_slow_emit(size_t ng, const uint32_t* __restrict__ gen,
                                                       const uint32_t* __restrict__ list,
                                                       const uint32_t* __restrict__ nbr,
                                                       const uint8_t* __restrict__ blevel,
@@ -487,14 +491,18 @@ __global__ void __launch_bounds__(256, 4) k_slow_emit(size_t ng, const uint32_t*
         if (t < 104) {
             uint32_t nb = nbr[(size_t)b * 104 + t];
             T.nbr[t] = nb;
-            T.nlv[t] = nb == FL_INVALID_INDEX ? 0xFF : blevel[nb];
+            const bool has = nb != FL_INVALID_INDEX;
+            T.nlv[t] = has ? blevel[nb] : 0xFF;
+            T.org[t][0] = has ? bx[nb] * 8 : 0;
+            T.org[t][1] = has ? by[nb] * 8 : 0;
+            T.org[t][2] = has ? bz[nb] * 8 : 0;
         }
-        if (t < 128) Qm[t] = qmask[(size_t)b * 128 + t];
-        if (t >= 128 && t < 160) T.solid[t - 128] = hsolid[(size_t)b * 32 + (t - 128)];
-        if (t == 160) T.near = brick_near_sphere(c, bx[b], by[b], bz[b], l) | (mnear ? mnear[b] & 1 : 0);
+        Qm[t] = qmask[(size_t)b * 128 + t];
+        if (t < 32) T.solid[t] = hsolid[(size_t)b * 32 + t];
+        if (t == 127) T.near = brick_near_sphere(c, bx[b], by[b], bz[b], l) | (mnear ? mnear[b] & 1 : 0);
         const uint32_t total = cnt[p];
         uint64_t* out = desc + off[p];
-        const int64_t G0[3] = {(int64_t)bx[b] * 8, (int64_t)by[b] * 8, (int64_t)bz[b] * 8};
+        const int32_t G0[3] = {bx[b] * 8, by[b] * 8, bz[b] * 8};
         __syncthreads();
         for (uint32_t k = t; k < total; k += blockDim.x) {
             int lo = 0, hi = 127;
@@ -505,24 +513,34 @@ __global__ void __launch_bounds__(256, 4) k_slow_emit(size_t ng, const uint32_t*
             }
             const uint4 w = Qm[lo];
             uint32_t r = k - w.w;
-            int q = 1, i = 0;
-            for (; q < Q; ++q) {
-                const uint32_t word = (q >> 3) == 0 ? w.x : ((q >> 3) == 1 ? w.y : w.z);
-                const uint32_t nib = (word >> ((q & 7) * 4)) & 0xFu;
-                const uint32_t cq = __popc(nib);
-                if (r < cq) {
-                    uint32_t v = nib;
-                    for (uint32_t skip = 0; skip < r; ++skip) v &= v - 1u;
-                    i = __ffs(v) - 1;
-                    break;
+            // the r-th set bit of the quad's 76: its word, then its byte, then its place there
+            uint32_t word = w.x;
+            int bit = 0;
+            if (r >= (uint32_t)__popc(w.x)) {
+                r -= __popc(w.x);
+                word = w.y;
+                bit = 32;
+                if (r >= (uint32_t)__popc(w.y)) {
+                    r -= __popc(w.y);
+                    word = w.z;
+                    bit = 64;
                 }
-                r -= cq;
             }
-            if (q >= Q) {  // the quad masks do not hold k (not reached when they match cnt)
+#pragma unroll
+            for (int byte = 0; byte < 3; ++byte) {
+                const uint32_t c8 = __popc(word & 0xFFu);
+                if (r < c8) break;
+                r -= c8;
+                word >>= 8;
+                bit += 8;
+            }
+            for (; r > 0; --r) word &= word - 1u;
+            bit += __ffs(word) - 1;
+            if (word == 0u || bit >= 4 * Q) {  // the quad masks do not hold k (not reached when they match cnt)
                 atomicAdd(dev_status + FL_DEVSTAT_BOUNDS, 1u);
-                q = 0;
+                bit = 0;
             }
-            out[k] = resolve_source(c, bx, by, bz, b, q, l, lo * 4 + i, G0, T, dev_status);
+            out[k] = resolve_source(c, b, bit >> 2, l, lo * 4 + (bit & 3), G0, T, dev_status);
         }
         __syncthreads();
     }
@@ -906,15 +924,15 @@ __global__ void k_mask_near(size_t n, const uint8_t* __restrict__ blevel, const 
             continue;
         }
         const int l = blevel[b];
-        const int64_t G0[3] = {(int64_t)bx[b] * 8, (int64_t)by[b] * 8, (int64_t)bz[b] * 8};
+        const int32_t G0[3] = {bx[b] * 8, by[b] * 8, bz[b] * 8};
         bool any = false, all = true;
         for (int i = lane; i < 1000; i += 32) {
             const int h[3] = {i % 10, (i / 10) % 10, i / 100};
-            int64_t G[3];
+            int32_t G[3];
             for (int ax = 0; ax < 3; ++ax) {
                 G[ax] = G0[ax] + h[ax] - 1;
                 if (!c.periodic[ax]) continue;
-                const int64_t N = ((int64_t)c.ext[ax] * 8) << l;
+                const int32_t N = (c.ext[ax] * 8) << l;
                 G[ax] = G[ax] < 0 ? G[ax] + N : (G[ax] >= N ? G[ax] - N : G[ax]);
             }
             const bool sol = solid_at(c, G[0], G[1], G[2], l);
@@ -939,7 +957,9 @@ __global__ void k_mask_near(size_t n, const uint8_t* __restrict__ blevel, const 
 // (smask, 16), per x-quad the 76 bits "element (q, site) needs a descriptor"
 // (bit 4q + i) with the quad's first descriptor (qmask, 128 entries, in site
 // order), the descriptor count (cnt, by brick) and the fluid sites.  Lane L
-// owns sites 16L .. 16L + 15, i.e. the quads 4L .. 4L + 3.  Own sites inside
+// owns sites 16L .. 16L + 15, i.e. the quads 4L .. 4L + 3, as two rows of eight
+// whose bits are worked out together (25,065 bricks: 95 us a site and population
+// at a time, 33 a row).  Own sites inside
 // a solid get no descriptors: their relaxation ignores what they pulled.
 __global__ void __launch_bounds__(256) k_brick_table(size_t n, const uint32_t* __restrict__ nbr,
                                                      const uint8_t* __restrict__ blevel,
@@ -978,25 +998,24 @@ __global__ void __launch_bounds__(256) k_brick_table(size_t n, const uint32_t* _
             } else {
                 bool mine = c.has_sphere != 0;
                 for (int s = lane; s < 512 && mine; s += 32)
-                    mine = solid_at(c, (int64_t)bx[b] * 8 + (s & 7), (int64_t)by[b] * 8 + ((s >> 3) & 7),
-                                    (int64_t)bz[b] * 8 + (s >> 6), l);
+                    mine = solid_at(c, bx[b] * 8 + (s & 7), by[b] * 8 + ((s >> 3) & 7), bz[b] * 8 + (s >> 6), l);
                 all = __all_sync(0xFFFFFFFFu, mine);
             }
             if (all) general = 2;
         }
         if (lane == 0) bclass[b] = (uint8_t)general;
         if (general != 1) continue;  // uniform over the warp
-        const int64_t G0[3] = {(int64_t)bx[b] * 8, (int64_t)by[b] * 8, (int64_t)bz[b] * 8};
+        const int32_t G0[3] = {bx[b] * 8, by[b] * 8, bz[b] * 8};
         uint32_t word = 0;  // word `lane` of the 10^3 halo bits
         if (near) {
             for (int k = 0; k < 32; ++k) {
                 const int i = 32 * k + lane;
                 bool sd = false;
                 if (i < 1000) {
-                    int64_t G[3] = {G0[0] + i % 10 - 1, G0[1] + (i / 10) % 10 - 1, G0[2] + i / 100 - 1};
+                    int32_t G[3] = {G0[0] + i % 10 - 1, G0[1] + (i / 10) % 10 - 1, G0[2] + i / 100 - 1};
                     for (int ax = 0; ax < 3; ++ax) {
                         if (!c.periodic[ax]) continue;
-                        const int64_t N = ((int64_t)c.ext[ax] * 8) << l;
+                        const int32_t N = (c.ext[ax] * 8) << l;
                         G[ax] = G[ax] < 0 ? G[ax] + N : (G[ax] >= N ? G[ax] - N : G[ax]);
                     }
                     sd = solid_at(c, G[0], G[1], G[2], l);
@@ -1011,33 +1030,38 @@ __global__ void __launch_bounds__(256) k_brick_table(size_t n, const uint32_t* _
         const int z = lane >> 2, y0 = 2 * (lane & 3);
         uint32_t* W = s_wq[(threadIdx.x >> 5) & 7] + lane * 12;  // this lane's 4 quads x 3 mask words
         uint32_t mine = 0, own16 = 0, qcs = 0;                    // qcs: per-quad counts (<= 72), a byte each
+        // a row of eight sites at a time: per population the row its sources lie in, as eight bits --
+        // missing same-level neighbours of the row, its x faces apart, or its solid sites moved by c_x
+        auto halo = [&](int hy, int hz) -> uint32_t {  // the ten solid bits of a row of the halo
+            const int at = 10 * hy + 100 * hz;
+            return __funnelshift_r(S[at >> 5], S[(at >> 5) + 1], at & 31) & 0x3FFu;
+        };
 #pragma unroll 1
-        for (int u = 0; u < 4; ++u) {  // quad 4L + u: row y0 + (u >> 1), x = 4 (u & 1) .. + 3
+        for (int u = 0; u < 4; u += 2) {  // the quads 4L + u, 4L + u + 1 of row y0 + u / 2
             const int y = y0 + (u >> 1);
-            uint32_t w0 = 0u, w1 = 0u, w2 = 0u, qc = 0u;
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                const int x = 4 * (u & 1) + k;
-                const bool own_solid = near && solid_bit(S, x, y, z);
-                own16 |= (uint32_t)own_solid << (4 * u + k);
-                if (own_solid) continue;
+            const uint32_t own8 = near ? (halo(y + 1, z + 1) >> 1) & 0xFFu : 0u;
+            uint32_t wq[2][3] = {{0u, 0u, 0u}, {0u, 0u, 0u}}, qc[2] = {0u, 0u};
+            own16 |= own8 << (4 * u);
 #pragma unroll
-                for (int q = 1; q < Q; ++q) {
-                    const int xi = x - CXq(q), yi = y - CYq(q), zi = z - CZq(q);
-                    const int dir = ((zi >> 3) + 1) * 9 + ((yi >> 3) + 1) * 3 + ((xi >> 3) + 1);
-                    const bool sl = ((slow_dirs >> dir) & 1u) || (near && solid_bit(S, xi, yi, zi));
-                    const uint32_t bit = (uint32_t)sl << ((q & 7) * 4 + k);  // bit 4q + k of the 96
-                    if ((q >> 3) == 0) w0 |= bit;
-                    else if ((q >> 3) == 1) w1 |= bit;
-                    else w2 |= bit;
-                    qc += sl ? 1u : 0u;
-                }
+            for (int q = 1; q < Q; ++q) {
+                const int cx = CXq(q), yi = y - CYq(q), zi = z - CZq(q);
+                const int dir = ((zi >> 3) + 1) * 9 + ((yi >> 3) + 1) * 3;
+                uint32_t m = (slow_dirs >> (dir + 1)) & 1u ? 0xFFu : 0u;
+                if (cx == 1) m = (m & 0xFEu) | ((slow_dirs >> dir) & 1u);
+                if (cx == -1) m = (m & 0x7Fu) | (((slow_dirs >> (dir + 2)) & 1u) << 7);
+                if (near) m |= (halo(yi + 1, zi + 1) >> (1 - cx)) & 0xFFu;
+                m &= ~own8;  // sites inside a solid pull nothing that counts
+                wq[0][q >> 3] |= (m & 15u) << ((q & 7) * 4);  // bit 4q + k of the 96
+                wq[1][q >> 3] |= (m >> 4) << ((q & 7) * 4);
+                qc[0] += __popc(m & 15u);
+                qc[1] += __popc(m >> 4);
             }
-            W[3 * u] = w0;
-            W[3 * u + 1] = w1;
-            W[3 * u + 2] = w2;
-            qcs |= qc << (8 * u);
-            mine += qc;
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                for (int k = 0; k < 3; ++k) W[3 * (u + v) + k] = wq[v][k];
+                qcs |= qc[v] << (8 * (u + v));
+                mine += qc[v];
+            }
         }
         uint32_t incl = mine;
 #pragma unroll
@@ -1983,8 +2007,8 @@ int pool_topology_build(fl_ctx* ctx, fl_pool* P) {
         P->desc_cap = want;
     }
     if (ng) {
-        const unsigned egrid = (unsigned)std::min<size_t>(ng, (size_t)ctx->num_sms * 4);
-        k_slow_emit<<<egrid, 256, 0, ctx->stream>>>(ng, d_gen, P->list, P->nbr, P->mesh.level, P->mesh.x, P->mesh.y,
+        const unsigned egrid = (unsigned)std::min<size_t>(ng, (size_t)ctx->num_sms * kEmitCtas);
+        k_slow_emit<<<egrid, 128, 0, ctx->stream>>>(ng, d_gen, P->list, P->nbr, P->mesh.level, P->mesh.x, P->mesh.y,
                                                     P->mesh.z, P->mesh.case_id, P->d_cases, mnear, P->hsolid, P->qmask,
                                                     P->slow_cnt, P->slow_off, P->desc, ctx->dev_status);
         FL_CHECK_LAUNCH(ctx, "k_slow_emit");
@@ -2069,7 +2093,8 @@ int pool_regrid(fl_ctx* ctx, fl_pool* P, int use_vorticity, fl_adapt_stats* st, 
     }
     size_t M = 0;
     fl_adapt_stats s{};
-    rc = fl_adapt_prepare(ctx, &P->mesh, &cfg, dom, true, P->adapt_scratch, &M, &s, P->maxL);
+    // the pool's bricks are in key order unless this regrid is the one that sorts them
+    rc = fl_adapt_prepare(ctx, &P->mesh, &cfg, dom, true, P->adapt_scratch, &M, &s, P->maxL, use_vorticity >= 0);
     if (rc) return rc;
     // Nothing splits and nothing merges: the bricks, their key order, the tables
     // and the populations all stay as they are (AdaptationEngine.cpp:72-78 returns
