@@ -1545,6 +1545,79 @@ __global__ void k_blob_flags(fl_mesh_dev m, const float* __restrict__ blobs, int
     }
 }
 
+// The same flags from a cheaper sum where that settles them.  A thread takes kBlobCells cells; per
+// blob and cell the argument by FMA and one ex2.approx instead of the written-out exp (about 10
+// instructions for 45).  With amplitudes >= 0 (sum A) and n blobs the two sums differ by at most
+//   A * 9e-7 (relative error of the argument 6e-7, times e^-x x <= 0.37; both exponentials 6e-7)
+//   + 2 n 2^-24 v (rounding of both sums, whose terms are >= 0),
+// and the kernel allows e0 = 4e-6 A and e1 = 1.5e-7 n per v: a cell whose sum lies that close to a
+// threshold (one in a few thousand) is worked out again by the exact sum, so the flags are the same.
+// Bound by instruction issue: 25 M leaves, 48 blobs, 1,370 -> 372 us.
+constexpr int kBlobCells = 4;
+
+__global__ void __launch_bounds__(256) k_blob_flags_near(fl_mesh_dev m, const float* __restrict__ blobs, int nblobs,
+                                                         float lo, float hi, int max_level, float e0, float e1,
+                                                         int32_t* __restrict__ flags) {
+    extern __shared__ __align__(16) float sb[];
+    float4* fast = (float4*)sb;          // cx, cy, cz, -log2(e) / (2 sigma^2)
+    float* amp = sb + 4 * nblobs;        // amplitudes
+    for (int i = threadIdx.x; i < nblobs; i += blockDim.x) {
+        fast[i] = make_float4(blobs[5 * i], blobs[5 * i + 1], blobs[5 * i + 2], -1.44269504f * blobs[5 * i + 3]);
+        amp[i] = blobs[5 * i + 4];
+    }
+    __syncthreads();
+    const size_t step = (size_t)gridDim.x * blockDim.x * kBlobCells;
+    for (size_t base = (size_t)blockIdx.x * blockDim.x * kBlobCells + threadIdx.x; base < m.n; base += step) {
+        float px[kBlobCells], py[kBlobCells], pz[kBlobCells], v[kBlobCells];
+        int l[kBlobCells];
+#pragma unroll
+        for (int u = 0; u < kBlobCells; ++u) {
+            const size_t i = base + u * 256;
+            l[u] = i < m.n ? m.level[i] : 0;
+            const float inv = 1.0f / (float)(1 << l[u]);
+            px[u] = i < m.n ? ((float)m.x[i] + 0.5f) * inv : 0.0f;
+            py[u] = i < m.n ? ((float)m.y[i] + 0.5f) * inv : 0.0f;
+            pz[u] = i < m.n ? ((float)m.z[i] + 0.5f) * inv : 0.0f;
+            v[u] = 0.0f;
+        }
+        for (int k = 0; k < nblobs; ++k) {
+            const float4 B = fast[k];
+            const float A = amp[k];
+#pragma unroll
+            for (int u = 0; u < kBlobCells; ++u) {
+                const float dx = px[u] - B.x, dy = py[u] - B.y, dz = pz[u] - B.z;
+                const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
+                float e;
+                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(d2 * B.w));
+                v[u] = __fmaf_rn(A, e, v[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kBlobCells; ++u) {
+            const size_t i = base + u * 256;
+            if (i >= m.n) continue;
+            const float allow = __fmaf_rn(e1, v[u], e0);
+            if (fabsf(v[u] - hi) <= allow || fabsf(v[u] - lo) <= allow) {
+                float w = 0.0f;
+                for (int k = 0; k < nblobs; ++k) {
+                    const float* B = blobs + 5 * k;
+                    float dx = px[u] - B[0], dy = py[u] - B[1], dz = pz[u] - B[2];
+                    float d2 = dx * dx;
+                    d2 = d2 + dy * dy;
+                    d2 = d2 + dz * dz;
+                    float e = fl_exp_neg(-(d2 * B[3]));
+                    w = w + B[4] * e;
+                }
+                v[u] = w;
+            }
+            int32_t f = 0;
+            if (v[u] > hi && l[u] < max_level) f = 1;
+            else if (v[u] < lo) f = -1;
+            flags[i] = f;
+        }
+    }
+}
+
 }  // namespace
 
 extern "C" int fl_flags_from_blobs(fl_ctx* ctx, fl_mesh* mesh, const float* blobs_host, int nblobs, float lo, float hi,
@@ -1557,6 +1630,23 @@ extern "C" int fl_flags_from_blobs(fl_ctx* ctx, fl_mesh* mesh, const float* blob
                 "blobs");
     fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material, mesh->case_id,
                    mesh->num_cells};
+    // the near sum's bound holds for decaying blobs of amplitude >= 0 around the unit cube
+    bool near = lo > -1e30f && lo < 1e30f && hi > -1e30f && hi < 1e30f;
+    double amps = 0.0;
+    for (int k = 0; k < nblobs; ++k) {
+        const float* B = blobs_host + 5 * k;
+        for (int a = 0; a < 3; ++a) near = near && B[a] >= -1e3f && B[a] <= 1e3f;
+        near = near && B[3] >= 0.0f && B[3] <= 1e30f && B[4] >= 0.0f && B[4] <= 1e6f;
+        amps += (double)B[4];
+    }
+    if (near) {
+        k_blob_flags_near<<<fl_blocks((mesh->num_cells + kBlobCells - 1) / kBlobCells, 256, ctx->num_sms * 8), 256,
+                            (size_t)nblobs * 20, ctx->stream>>>(md, (const float*)ctx->scratch, nblobs, lo, hi, max_level,
+                                                                (float)(4e-6 * amps), 1.5e-7f * (float)nblobs,
+                                                                mesh->flags);
+        FL_CHECK_LAUNCH(ctx, "k_blob_flags_near");
+        return FL_OK;
+    }
     k_blob_flags<<<fl_blocks(mesh->num_cells, 256, ctx->num_sms * 8), 256, (size_t)nblobs * 20, ctx->stream>>>(
         md, (const float*)ctx->scratch, nblobs, 0, lo, hi, max_level, mesh->flags);
     FL_CHECK_LAUNCH(ctx, "k_blob_flags");
