@@ -318,7 +318,7 @@ __device__ __forceinline__ uint32_t sibling_in_run(const fl_probe& P, const fl_m
 // probe points tried.  Same answer as the 98 probes, from 56 on a filled mesh.
 __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom, fl_locator L, int min_level,
                                                 int check26, const uint8_t* __restrict__ shadow,
-                                                uint32_t* __restrict__ is_leader) {
+                                                uint32_t* __restrict__ is_leader, uint32_t* __restrict__ group_of) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
     __shared__ uint8_t surf[56];  // the outside cells k = ux + 4 uy + 16 uz of the 4^3 grid of child-sized cells
@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
         const size_t mine = base + lane;
         const bool cand = mine < m.n && merge_candidate(m, mine, min_level);
         if (mine < m.n && !cand) is_leader[mine] = 0u;
+        if (mine < m.n) group_of[mine] = FL_INVALID_INDEX;  // k_members fills in the groups
         unsigned cm = __ballot_sync(0xFFFFFFFFu, cand);
         while (cm) {
             const int n4 = min(__popc(cm), 4);  // candidates of this round
@@ -464,19 +465,49 @@ __global__ void __launch_bounds__(kT) k_members(fl_mesh_dev m, fl_domain_dev dom
 }
 
 // Output count per old cell, in visiting order (order[t] = the cell visited
-// t-th, or t when order is null).
-__global__ void k_counts(fl_mesh_dev m, int max_level, const uint32_t* __restrict__ order,
-                         const uint32_t* __restrict__ is_leader, const uint32_t* __restrict__ group_of,
-                         uint32_t* __restrict__ cnt) {
+// t-th, or t when order is null), and the split and surviving cells counted
+// (counters[4], [5]; one atomic each per block).
+__global__ void __launch_bounds__(kT) k_counts(fl_mesh_dev m, int max_level, const uint32_t* __restrict__ order,
+                                               const uint32_t* __restrict__ is_leader,
+                                               const uint32_t* __restrict__ group_of, uint32_t* __restrict__ cnt,
+                                               uint32_t* __restrict__ counters) {
+    __shared__ uint32_t s_sum[2];
+    if (threadIdx.x < 2) s_sum[threadIdx.x] = 0u;
+    __syncthreads();
     size_t stride = (size_t)gridDim.x * blockDim.x;
+    uint32_t ns = 0, nv = 0;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < m.n; t += stride) {
         const size_t i = order ? order[t] : t;
-        bool split = m.flags[i] > 0 && m.state[i] == 0 && m.level[i] < max_level;
-        uint32_t c;
-        if (split) c = 8;
-        else if (group_of[i] != FL_INVALID_INDEX) c = is_leader[i] ? 1u : 0u;
-        else c = 1;
-        cnt[t] = c;
+        const bool split = m.flags[i] > 0 && m.state[i] == 0 && m.level[i] < max_level;
+        const bool grouped = group_of[i] != FL_INVALID_INDEX;
+        ns += split ? 1u : 0u;
+        nv += !split && !grouped ? 1u : 0u;
+        cnt[t] = split ? 8u : (grouped ? (is_leader[i] ? 1u : 0u) : 1u);
+    }
+    ns = __reduce_add_sync(0xFFFFFFFFu, ns);
+    nv = __reduce_add_sync(0xFFFFFFFFu, nv);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(s_sum, ns);
+        atomicAdd(s_sum + 1, nv);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 && s_sum[threadIdx.x]) atomicAdd(counters + 4 + threadIdx.x, s_sum[threadIdx.x]);
+}
+
+// The fields of new cell j: copied from its source cell i, or the mean of group g's members (kind 2).
+__device__ __forceinline__ void emit_row(int kind, size_t i, uint32_t j, uint32_t g, const uint32_t* members,
+                                         const float* fin, float* fout, uint32_t C, int rule) {
+    float* fo = fout + (size_t)j * C;
+    if (kind != 2) {
+        const float* sp = fin + i * C;
+        for (uint32_t c = 0; c < C; ++c) fo[c] = sp[c];
+        return;
+    }
+    const uint32_t* mem = members + (size_t)g * 8;
+    for (uint32_t c = 0; c < C; ++c) {
+        float sum = 0.0f;
+        for (int q = 0; q < 8; ++q) sum = __fadd_rn(sum, fin[(size_t)mem[q] * C + c]);
+        fo[c] = rule == 1 ? sum : __fmul_rn(sum, 0.125f);
     }
 }
 
@@ -489,6 +520,63 @@ __global__ void k_counts(fl_mesh_dev m, int max_level, const uint32_t* __restric
 // emit nothing).  Fields (C per cell, AoS) follow the reference: children copy
 // their parent (prolongation), a parent sums its children 0..7 in order, x0.125
 // for the arithmetic rule (restriction).
+//
+// Groups of 32 cells without a split cell, most of them in a regrid that
+// follows a moving feature: each cell makes at most one, neighbouring lanes
+// neighbouring ones, so a cell's columns are loaded together and go straight
+// out.  The other groups go into list for k_emit.  25 M cells of which a few
+// per cent change: 492 us for all groups in k_emit (64 registers, three
+// dependent loads a cell), 161 for both.
+__global__ void __launch_bounds__(kT, 8) k_emit_plain(fl_mesh_dev m, int max_level, const uint32_t* __restrict__ order,
+                                                      const uint32_t* __restrict__ off,
+                                                      const uint32_t* __restrict__ is_leader,
+                                                      const uint32_t* __restrict__ group_of,
+                                                      const uint32_t* __restrict__ members, fl_mesh_out out,
+                                                      uint32_t* __restrict__ osrc, uint8_t* __restrict__ okind,
+                                                      const float* __restrict__ fin, float* __restrict__ fout, uint32_t C,
+                                                      int rule, uint32_t* __restrict__ list, uint32_t* __restrict__ list_n) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < m.n; t0 += stride) {
+        const size_t t = t0 + lane;
+        const bool in = t < m.n;
+        const size_t i = in ? (order ? order[t] : t) : 0;
+        const int32_t x = m.x[i], y = m.y[i], z = m.z[i], fl = m.flags[i];
+        const int l = m.level[i];
+        const uint8_t state = m.state[i];
+        const uint32_t material = m.material[i], g = group_of[i], o = in ? off[t] : 0u;
+        if (__any_sync(0xFFFFFFFFu, in && fl > 0 && state == 0 && l < max_level)) {
+            if (lane == 0) list[atomicAdd(list_n, 1u)] = (uint32_t)(t0 >> 5);
+            continue;
+        }
+        const bool grouped = g != FL_INVALID_INDEX;
+        const bool makes = in && (!grouped || is_leader[i]);
+        if (makes) {
+            const int up = grouped ? 1 : 0;
+            out.x[o] = x >> up;
+            out.y[o] = y >> up;
+            out.z[o] = z >> up;
+            out.level[o] = (uint8_t)(l - up);
+            out.state[o] = state;
+            out.material[o] = material;
+            out.flags[o] = 0;
+            if (out.case_id) out.case_id[o] = m.case_id ? m.case_id[i] : 0;
+            if (osrc) osrc[o] = up ? g : (uint32_t)i;
+            if (okind) okind[o] = up ? 9 : 8;
+        }
+        if (fin && C) {
+            if (!order && __all_sync(0xFFFFFFFFu, makes && !grouped)) {  // 32 rows in one piece
+                const float* sp = fin + t0 * C;
+                float* fo = fout + (size_t)__shfl_sync(0xFFFFFFFFu, o, 0) * C;
+                for (uint32_t e = lane; e < 32u * C; e += 32u) fo[e] = sp[e];
+            } else if (makes) {
+                emit_row(grouped ? 2 : 3, i, o, g, members, fin, fout, C, rule);
+            }
+        }
+    }
+}
+
+// The groups with split cells: their new cells staged in shared memory, column by column.
 __global__ void __launch_bounds__(kT) k_emit(fl_mesh_dev m, fl_domain_dev dom, int max_level,
                                              const uint32_t* __restrict__ order, const uint32_t* __restrict__ off,
                                              const uint32_t* __restrict__ is_leader,
@@ -496,7 +584,8 @@ __global__ void __launch_bounds__(kT) k_emit(fl_mesh_dev m, fl_domain_dev dom, i
                                              const uint32_t* __restrict__ members, fl_mesh_out out,
                                              uint32_t* __restrict__ osrc, uint8_t* __restrict__ okind,
                                              const float* __restrict__ fin, float* __restrict__ fout, uint32_t C,
-                                             int rule) {
+                                             int rule, const uint32_t* __restrict__ list,
+                                             const uint32_t* __restrict__ list_n) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
     __shared__ uint32_t stage[kT / 32][256];  // one column of a warp's (at most 256) new cells
@@ -504,10 +593,9 @@ __global__ void __launch_bounds__(kT) k_emit(fl_mesh_dev m, fl_domain_dev dom, i
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t* S = stage[threadIdx.x >> 5];
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    const size_t rounds = (m.n + stride - 1) / stride;  // whole warps stay in the loop
-    for (size_t rr = 0; rr < rounds; ++rr) {
-        const size_t t = rr * stride + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t groups = *list_n, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < groups; w += warps) {
+        const size_t t = (size_t)list[w] * 32 + lane;
         // kind: 0 nothing (a merged non-leader or past the end), 1 split, 2 group leader, 3 kept
         int kind = 0, l = 0;
         size_t i = 0;
@@ -585,24 +673,11 @@ __global__ void __launch_bounds__(kT) k_emit(fl_mesh_dev m, fl_domain_dev dom, i
             for (uint32_t e = lane; e < total; e += 32u) okind[base + e] = (uint8_t)S[e];
             __syncwarp();
         }
-        if (fin && C && kind) {  // fields: copied from the source cell, or the mean of a group's members
-            auto copy_row = [&](uint32_t j) {
-                const float* sp = fin + i * C;
-                float* fo = fout + (size_t)j * C;
-                for (uint32_t c = 0; c < C; ++c) fo[c] = sp[c];
-            };
+        if (fin && C) {
             if (kind == 1) {
-                for (int c = 0; c < 8; ++c) copy_row(o + (t1[st * 8 + c] & 7u));
-            } else if (kind == 3) {
-                copy_row(o);
-            } else {
-                const uint32_t* mem = members + (size_t)g * 8;
-                float* fo = fout + (size_t)o * C;
-                for (uint32_t c = 0; c < C; ++c) {
-                    float sum = 0.0f;
-                    for (int q = 0; q < 8; ++q) sum = __fadd_rn(sum, fin[(size_t)mem[q] * C + c]);
-                    fo[c] = rule == 1 ? sum : __fmul_rn(sum, 0.125f);
-                }
+                for (int c = 0; c < 8; ++c) emit_row(kind, i, o + (t1[st * 8 + c] & 7u), g, members, fin, fout, C, rule);
+            } else if (kind) {
+                emit_row(kind, i, o, g, members, fin, fout, C, rule);
             }
         }
     }
@@ -825,26 +900,14 @@ static AdaptWork carve_adapt(void* scratch, size_t n, bool with_case) {
     return w;
 }
 
-__global__ void k_count_kinds(fl_mesh_dev m, int max_level, const uint32_t* __restrict__ group_of,
-                              uint32_t* __restrict__ counters) {
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    uint32_t ns = 0, nv = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m.n; i += stride) {
-        bool split = m.flags[i] > 0 && m.state[i] == 0 && m.level[i] < max_level;
-        if (split) ++ns;
-        else if (group_of[i] == FL_INVALID_INDEX) ++nv;
-    }
-    if (ns) atomicAdd(counters + 4, ns);
-    if (nv) atomicAdd(counters + 5, nv);
-}
-
 // Phase 1: balance, classify, emit the unsorted new cell list; returns its size.
 int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const fl_domain_dev& dom,
                      bool run_balance, void* scratch, size_t* M_out, fl_adapt_stats* st, int level_bound,
-                     bool in_key_order) {
+                     bool in_key_order, const uint32_t** order) {
     size_t n = mesh->num_cells;
     fl_adapt_stats s{};
     *M_out = 0;
+    *order = nullptr;
     if (n == 0) { if (st) *st = s; return FL_OK; }
     AdaptWork w = carve_adapt(scratch, n, mesh->case_id != nullptr);
     fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material,
@@ -854,6 +917,7 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
     fl_locator L;
     int rc = fl_locator_build(ctx, md, dom, w.locator, &L, level_bound, in_key_order);
     if (rc) return rc;
+    *order = L.ids;
     if (run_balance && cfg->balance_mode == 0) {
         rc = fl_launch_cell_keys(ctx, mesh->x, mesh->y, mesh->z, mesh->level, mesh->case_id, dom.depth,
                                  dom.anchor_level, w.keys, n);
@@ -869,22 +933,22 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
         if (rc) return rc;
     }
     unsigned nb = fl_blocks(n, kT, ctx->num_sms * 8);
-    k_shadow_update<<<nb, kT, 0, ctx->stream>>>(md, 1, cfg->max_refinement_level, w.shadow, nullptr);  // final levels
-    FL_CHECK_LAUNCH(ctx, "k_shadow_update");
+    // the merge condition wants the levels the cells will have: FULL26 balance leaves them in
+    // w.shadow (no flag changes after its last update), and FACE6 merges do not ask
     int check26 = cfg->enforce_2_1_balance && cfg->balance_mode == 1;
+    if (check26 && !run_balance) {
+        k_shadow_update<<<nb, kT, 0, ctx->stream>>>(md, 1, cfg->max_refinement_level, w.shadow, nullptr);
+        FL_CHECK_LAUNCH(ctx, "k_shadow_update");
+    }
     const unsigned wb = fl_blocks((n + 31) / 32 * 32, kT, ctx->num_sms * 8);  // a warp per 32 cells
-    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, check26, w.shadow, w.leader);
+    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, check26, w.shadow, w.leader, w.group_of);
     FL_CHECK_LAUNCH(ctx, "k_leaders");
     rc = fl_scan_u32_with(ctx, w.leader, w.gid, n, w.counters + 2, w.scan_scratch);
     if (rc) return rc;
-    rc = fl_launch_fill_u32(ctx, w.group_of, FL_INVALID_INDEX, n);
-    if (rc) return rc;
     k_members<<<wb, kT, 0, ctx->stream>>>(md, dom, L, w.leader, w.gid, w.members, w.group_of);
     FL_CHECK_LAUNCH(ctx, "k_members");
-    k_counts<<<nb, kT, 0, ctx->stream>>>(md, cfg->max_refinement_level, L.ids, w.leader, w.group_of, w.cnt);
+    k_counts<<<nb, kT, 0, ctx->stream>>>(md, cfg->max_refinement_level, L.ids, w.leader, w.group_of, w.cnt, w.counters);
     FL_CHECK_LAUNCH(ctx, "k_counts");
-    k_count_kinds<<<nb, kT, 0, ctx->stream>>>(md, cfg->max_refinement_level, w.group_of, w.counters);
-    FL_CHECK_LAUNCH(ctx, "k_count_kinds");
     rc = fl_scan_u32_with(ctx, w.cnt, w.cnt, n, w.counters + 3, w.scan_scratch);
     if (rc) return rc;
     uint32_t hc[6] = {0, 0, 0, 0, 0, 0};
@@ -906,8 +970,8 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
 
 // Phase 2: the new cells straight into `out` (capacity >= M), in key order.
 int fl_adapt_finish(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const fl_domain_dev& dom,
-                    void* scratch, size_t M, const float* fields, uint32_t C, fl_mesh* out, float* out_fields,
-                    uint32_t* osrc, uint8_t* okind, uint32_t* omembers, uint32_t num_groups) {
+                    void* scratch, const uint32_t* order, size_t M, const float* fields, uint32_t C, fl_mesh* out,
+                    float* out_fields, uint32_t* osrc, uint8_t* okind, uint32_t* omembers, uint32_t num_groups) {
     size_t n = mesh->num_cells;
     if (n == 0 || M == 0) return FL_OK;
     AdaptWork w = carve_adapt(scratch, n, mesh->case_id != nullptr);
@@ -915,9 +979,15 @@ int fl_adapt_finish(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg
                    mesh->case_id, n};
     fl_mesh_out o{out->x, out->y, out->z, out->level, out->state, out->flags, out->material,
                   mesh->case_id ? out->case_id : nullptr};
+    uint32_t* list = (uint32_t*)w.viol;      // groups of 32 cells: n / 8 of the balance's n bytes
+    uint32_t* list_n = w.counters + 6;       // still 0
+    k_emit_plain<<<fl_blocks(n, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(
+        md, cfg->max_refinement_level, order, w.cnt, w.leader, w.group_of, w.members, o, osrc, okind, fields, out_fields,
+        C, cfg->averaging_rule, list, list_n);
+    FL_CHECK_LAUNCH(ctx, "k_emit_plain");
     k_emit<<<fl_blocks(n, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(
-        md, dom, cfg->max_refinement_level, fl_locator_ids(w.locator, n), w.cnt, w.leader, w.group_of, w.members, o,
-        osrc, okind, fields, out_fields, C, cfg->averaging_rule);
+        md, dom, cfg->max_refinement_level, order, w.cnt, w.leader, w.group_of, w.members, o, osrc, okind, fields,
+        out_fields, C, cfg->averaging_rule, list, list_n);
     FL_CHECK_LAUNCH(ctx, "k_emit");
     if (omembers && num_groups)
         FL_TRY_CUDA(ctx, cudaMemcpyAsync(omembers, w.members, (size_t)num_groups * 32, cudaMemcpyDeviceToDevice,
@@ -1020,7 +1090,7 @@ int fl_neighbour_rebuild(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config
     bool done = false;
     rc = fl_neighbours_octree(ctx, md, dom, ext, subslots, cv.p, nbr, &done);
     if (rc) return rc;
-    if (done) return fl_collect_device_status(ctx, "fl_neighbour_rebuild");
+    if (done) return FL_OK;
     uint32_t* marks = cv.take<uint32_t>(n);
     fl_locator L;
     rc = fl_locator_build(ctx, md, dom, cv.p, &L);
@@ -1049,7 +1119,8 @@ int fl_adapt(fl_ctx* ctx, fl_mesh* mesh, const fl_adapt_config* cfg, float** fie
     dom.max_level = cfg->max_refinement_level > 0 ? cfg->max_refinement_level : dom.anchor_level;
     size_t M = 0;
     fl_adapt_stats s{};
-    rc = fl_adapt_prepare(ctx, mesh, cfg, dom, cfg->enforce_2_1_balance != 0, scratch, &M, &s);
+    const uint32_t* order = nullptr;
+    rc = fl_adapt_prepare(ctx, mesh, cfg, dom, cfg->enforce_2_1_balance != 0, scratch, &M, &s, -1, false, &order);
     if (rc) return rc;
     // no change: keep the buffers (AdaptationEngine.cpp:72-77), flags still reset below
     size_t cap_out = mesh->capacity;
@@ -1069,7 +1140,7 @@ int fl_adapt(fl_ctx* ctx, fl_mesh* mesh, const fl_adapt_config* cfg, float** fie
             return fl_check_cuda(ctx, e, "fields alloc");
         }
     }
-    rc = fl_adapt_finish(ctx, mesh, cfg, dom, scratch, M, C ? *fields : nullptr, C, &out, nf, nullptr, nullptr,
+    rc = fl_adapt_finish(ctx, mesh, cfg, dom, scratch, order, M, C ? *fields : nullptr, C, &out, nf, nullptr, nullptr,
                          nullptr, s.num_groups);
     if (rc) {
         fl_mesh_free(ctx, &out);
@@ -1153,11 +1224,9 @@ int fl_merge(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const
     rc = fl_locator_build(ctx, md, dom, loc, &L);
     if (rc) return rc;
     const unsigned wb = fl_blocks((n + 31) / 32 * 32, kT, ctx->num_sms * 8);  // a warp per 32 cells
-    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, 0, nullptr, leader);
+    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, 0, nullptr, leader, group_of);
     FL_CHECK_LAUNCH(ctx, "k_leaders");
     rc = fl_scan_u32_with(ctx, leader, gid, n, total, ss);
-    if (rc) return rc;
-    rc = fl_launch_fill_u32(ctx, group_of, FL_INVALID_INDEX, n);
     if (rc) return rc;
     k_members<<<wb, kT, 0, ctx->stream>>>(md, dom, L, leader, gid, members, group_of);
     FL_CHECK_LAUNCH(ctx, "k_members");

@@ -17,10 +17,11 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
                    uint8_t* shadow, uint8_t* viol, uint8_t* act, uint32_t* counters, fl_balance_result* res,
                    bool balanced_input = false);
 // level_bound >= 0: no cell of the mesh is deeper; in_key_order: its cells are in key order (the
-// point locator then skips a host read each).
+// point locator then skips a host read each).  *order: the cells in key order, in scratch, or
+// nullptr when the mesh is in key order; fl_adapt_finish takes it.
 int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const fl_domain_dev& dom,
-                     bool run_balance, void* scratch, size_t* M_out, fl_adapt_stats* st, int level_bound = -1,
-                     bool in_key_order = false);
+                     bool run_balance, void* scratch, size_t* M_out, fl_adapt_stats* st, int level_bound,
+                     bool in_key_order, const uint32_t** order);
 int fl_adapt_finish(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const fl_domain_dev& dom,
-                    void* scratch, size_t M, const float* fields, uint32_t C, fl_mesh* out, float* out_fields,
+                    void* scratch, const uint32_t* order, size_t M, const float* fields, uint32_t C, fl_mesh* out, float* out_fields,
                     uint32_t* osrc, uint8_t* okind, uint32_t* omembers, uint32_t num_groups);

@@ -15,6 +15,9 @@
 #include "keys.cuh"
 #include "scan.cuh"
 
+#include <algorithm>
+#include <cstring>
+
 namespace {
 
 constexpr int kProbeLimit = 256;
@@ -154,9 +157,9 @@ __global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__
 
 // Run start of every leaf divided by 8^cut: the anchor shifted down by cut,
 // encoded at depth - cut levels, the low 3(A - l - cut) bits cleared (the case
-// id above bit 3 * (depth - cut)); ids[i] = i.
+// id above bit 3 * (depth - cut)).
 __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev dom, int cut,
-                                                  uint64_t* __restrict__ keys, uint32_t* __restrict__ ids) {
+                                                  uint64_t* __restrict__ keys) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
@@ -170,8 +173,12 @@ __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev d
         k &= ~((1ull << (3 * (sh - cut))) - 1);
         if (m.case_id) k |= (uint64_t)m.case_id[i] << (3 * dc);
         keys[i] = k;
-        ids[i] = (uint32_t)i;
     }
+}
+
+__global__ void k_iota(uint32_t* __restrict__ ids, size_t n) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) ids[i] = (uint32_t)i;
 }
 
 // flag = 1 when some run start is smaller than the one before it.
@@ -599,8 +606,6 @@ size_t fl_locator_scratch_bytes(size_t n) {
     return fl_align256(n * 8) + fl_align256(n * 4) + fl_align256((nb + 1) * 4) + 256 + fl_sort_scratch_bytes(n, 8);
 }
 
-uint32_t* fl_locator_ids(void* scratch, size_t n) { return (uint32_t*)((char*)scratch + fl_align256(n * 8)); }
-
 int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom, void* scratch, fl_locator* L,
                      int level_bound, bool in_key_order) {
     const size_t n = m.n;
@@ -621,7 +626,7 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
         if (rc) return rc;
     }
     L->cut = dom.anchor_level > (int)hf[1] ? dom.anchor_level - (int)hf[1] : 0;
-    k_run_keys<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, dom, L->cut, keys, ids);
+    k_run_keys<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, dom, L->cut, keys);
     FL_CHECK_LAUNCH(ctx, "k_run_keys");
     hf[0] = 0;
     if (!in_key_order) {
@@ -631,6 +636,8 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
         if (rc) return rc;
     }
     if (hf[0]) {  // stable: equal run starts keep mesh order, so the last of them is found
+        k_iota<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(ids, n);
+        FL_CHECK_LAUNCH(ctx, "k_iota");
         // the keys hold 3 (depth - cut) bits, plus 16 for case ids
         const int end_bit = std::min(64, 3 * (dom.depth - L->cut) + (m.case_id ? 16 : 0));
         int rc = fl_sort_pairs_with(ctx, keys, ids, n, 0, end_bit, p);
@@ -734,9 +741,13 @@ int fl_neighbours_octree(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev&
         FL_CHECK_LAUNCH(ctx, "k_neighbours_nodes");
     }
     uint32_t st[4];
-    rc = fl_read_back(ctx, st, T.state, sizeof(st), "octree state");
-    *done = !rc && !st[0] && (!T.list || (size_t)st[2] + st[3] == n);
-    return rc;
+    rc = fl_read_enqueue(ctx, 0, T.state, sizeof(st), "octree state");
+    if (rc) return rc;
+    rc = fl_collect_device_status(ctx, "fl_neighbour_rebuild");  // waits for both reads
+    if (rc) return rc;
+    std::memcpy(st, ctx->host_read, sizeof(st));
+    *done = !st[0] && (!T.list || (size_t)st[2] + st[3] == n);
+    return FL_OK;
 }
 
 int fl_hash_lg(uint64_t cap) {

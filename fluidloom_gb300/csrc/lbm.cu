@@ -2183,8 +2183,9 @@ int pool_regrid(fl_ctx* ctx, fl_pool* P, int use_vorticity, fl_adapt_stats* st, 
     }
     size_t M = 0;
     fl_adapt_stats s{};
+    const uint32_t* order = nullptr;
     // the pool's bricks are in key order unless this regrid is the one that sorts them
-    rc = fl_adapt_prepare(ctx, &P->mesh, &cfg, dom, true, P->adapt_scratch, &M, &s, P->maxL, use_vorticity >= 0);
+    rc = fl_adapt_prepare(ctx, &P->mesh, &cfg, dom, true, P->adapt_scratch, &M, &s, P->maxL, use_vorticity >= 0, &order);
     if (rc) return rc;
     // Nothing splits and nothing merges: the bricks, their key order, the tables
     // and the populations all stay as they are (AdaptationEngine.cpp:72-78 returns
@@ -2226,8 +2227,8 @@ int pool_regrid(fl_ctx* ctx, fl_pool* P, int use_vorticity, fl_adapt_stats* st, 
         rc = alloc_brick_arrays_beside(ctx, P, new_cap, &fresh);
         if (rc) return undo(rc);
     }
-    rc = fl_adapt_finish(ctx, &P->mesh, &cfg, dom, P->adapt_scratch, M, nullptr, 0, &out, nullptr, osrc, okind, members,
-                         s.num_groups);
+    rc = fl_adapt_finish(ctx, &P->mesh, &cfg, dom, P->adapt_scratch, order, M, nullptr, 0, &out, nullptr, osrc, okind,
+                         members, s.num_groups);
     if (rc) return undo(rc);
     float* target = grew ? nf[0] : P->f[2];
     k_remap<<<fl_blocks(M * 512, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(view(P), M, osrc, okind, members,
