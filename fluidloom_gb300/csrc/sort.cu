@@ -5,7 +5,7 @@
 // whose atomic_inc scatter is unstable and whose digit is fixed at 8 bits,
 // radix_sort.cl:5-6).  Design (onesweep, Adinets & Merrill 2022):
 //  1. one upfront pass histograms every digit of every pass at once
-//     (per-CTA shared histograms, then global atomics), and one tiny kernel
+//     (per-CTA shared histograms, then global atomics), and its last block
 //     turns each pass histogram into exclusive bin offsets;
 //  2. per pass, one kernel: each CTA takes the next tile (atomic ticket), ranks
 //     its keys stably with warp __match_any_sync peer groups and per-warp
@@ -41,11 +41,15 @@ __host__ __device__ constexpr uint32_t digit_mask(int end_bit, int sh, int bits)
     return end_bit - sh >= bits ? (1u << bits) - 1u : (1u << (end_bit - sh)) - 1u;
 }
 
+// Every pass's histogram, then, in the block that finishes last (*done counts the
+// blocks, starting at 0), each pass's bins scanned in place to exclusive offsets: a
+// warp per pass, R / 32 consecutive bins a lane.
 template <int kBits>
 __global__ void __launch_bounds__(256) k_histogram(const uint64_t* __restrict__ keys, size_t n, int begin_bit,
-                                                   int end_bit, int passes, uint32_t* __restrict__ hist) {
+                                                   int end_bit, int passes, uint32_t* hist, unsigned* done) {
     constexpr int R = 1 << kBits;
     __shared__ uint32_t h[kMaxPasses][R];
+    __shared__ bool last;
     for (int i = threadIdx.x; i < kMaxPasses * R; i += blockDim.x) (&h[0][0])[i] = 0;
     __syncthreads();
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -61,24 +65,33 @@ __global__ void __launch_bounds__(256) k_histogram(const uint64_t* __restrict__ 
         uint32_t v = (&h[0][0])[i];
         if (v) atomicAdd(hist + i, v);
     }
-}
-
-// Exclusive scan of each pass's bins (one CTA of R threads per pass).
-template <int kBits>
-__global__ void k_bin_offsets(uint32_t* hist) {
-    constexpr int R = 1 << kBits;
-    __shared__ uint32_t s[R];
-    uint32_t* h = hist + blockIdx.x * R;
-    int t = threadIdx.x;
-    s[t] = h[t];
+    __threadfence();
     __syncthreads();
-    for (int o = 1; o < R; o <<= 1) {
-        uint32_t v = t >= o ? s[t - o] : 0u;
-        __syncthreads();
-        s[t] += v;
-        __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int lane = threadIdx.x & 31, p = threadIdx.x >> 5;  // 8 warps, at most 8 passes
+    if (p >= passes) return;
+    uint32_t* g = hist + p * R + lane * (R / 32);
+    uint32_t v[R / 32], sum = 0;
+#pragma unroll
+    for (int j = 0; j < R / 32; ++j) {
+        v[j] = __ldcg(g + j);
+        sum += v[j];
     }
-    h[t] = s[t] - h[t];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    uint32_t run = incl - sum;
+#pragma unroll
+    for (int j = 0; j < R / 32; ++j) {
+        g[j] = run;
+        run += v[j];
+    }
 }
 
 __device__ __forceinline__ uint32_t ld_vol(const uint32_t* p) { return *(volatile const uint32_t*)p; }
@@ -115,6 +128,10 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) { s_tile = (int)atomicAdd(ticket, 1u); s_bad = 0; }
     for (int i = threadIdx.x; i < kWarps * R; i += kThreads) s_warp_hist[i] = 0;
+    // the passes are launched programmatically: this much of a pass overlaps the one before it,
+    // whose output is read from here on
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     __syncthreads();
     const int tile = s_tile;
     const size_t tbase = (size_t)tile * kTile;
@@ -267,10 +284,11 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
 // A pass of one tile is a chain of latencies (about 11,800 cycles at 12 keys per thread: 4,000 rank
 // them, 1,800 stage them, 2,400 write them out), so while the tiles fit the GPU at once a sort takes
 // as long as one tile, and fewer keys per thread make more and shorter tiles.  Their look-back is
-// longer, so it reads kSmallWindow words per round trip.  Keys and sort, 12 -> 4 keys per thread:
-// 3,000 63-bit keys 84 -> 65 us, 40,961 30-bit keys 61 -> 51, 240,000 63-bit keys 128 -> 120,
-// 600,000 162 -> 158; at 1,000,000 the tiles no longer fit at once, 196 -> 214.
-constexpr size_t kSmallSort = 1u << 19;
+// longer, so it reads kSmallWindow words per round trip, and each pass starts while the one before
+// it ends.  Keys and sort: 40,961 30-bit keys 61 us with 12 keys per thread, 49 with 4, 37 with the
+// passes overlapped too; 3,000 63-bit keys 85 -> 42, 240,000 117 -> 89, 1,000,000 180 -> 176, and
+// 1,500,000, whose tiles no longer fit at once, 224 -> 225.
+constexpr size_t kSmallSort = 1u << 20;
 
 // Bytes of one pass's tile status words and ticket, for every shape: at most
 // ceil(n / smallest tile) tiles of at most kMaxRadix digits (9-bit digits on the
@@ -282,7 +300,7 @@ size_t status_stride_min(size_t n) {
 
 // All passes of one shape.  The scratch layout (fl_sort_scratch_bytes): the
 // alternate key and value buffers, the pass histograms (kMaxPasses x
-// kMaxRadix), then per pass its tile status words and ticket, at a stride that
+// kMaxRadix), a block count, then per pass its tile status words and ticket, at a stride that
 // fits every shape's tiles (status_stride_min).
 template <int kThreads, int kBits, int kItems>
 int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin_bit, int end_bit, void* scratch) {
@@ -295,19 +313,28 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
     uint64_t* kalt = (uint64_t*)p; p += fl_align256(n * 8);
     uint32_t* valt = (uint32_t*)p; p += fl_align256(n * 4);
     uint32_t* hist = (uint32_t*)p; p += fl_align256((size_t)kMaxPasses * kMaxRadix * 4);
+    unsigned* done = (unsigned*)p; p += 256;
     char* stat0 = p;
     const size_t stat_stride = fl_align256(tiles * R * 4 + 4);  // at most status_stride_min(n)
-    // clear histograms + per-pass status/tickets in one memset
-    FL_TRY_CUDA(ctx, cudaMemsetAsync(hist, 0, fl_align256((size_t)kMaxPasses * kMaxRadix * 4) + passes * stat_stride,
+    // clear histograms, their block count and the per-pass status/tickets in one memset
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(hist, 0, fl_align256((size_t)kMaxPasses * kMaxRadix * 4) + 256 + passes * stat_stride,
                                      ctx->stream), "sort clear");
     constexpr size_t smem = onesweep_smem<kThreads, kBits, kItems>();
     FL_TRY_CUDA(ctx, cudaFuncSetAttribute(k_onesweep<kThreads, kBits, kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem), "sort shared memory");
     unsigned hb = fl_blocks(n, 256, ctx->num_sms * 4);
-    k_histogram<kBits><<<hb, 256, 0, ctx->stream>>>(keys, n, begin_bit, end_bit, passes, hist);
+    k_histogram<kBits><<<hb, 256, 0, ctx->stream>>>(keys, n, begin_bit, end_bit, passes, hist, done);
     FL_CHECK_LAUNCH(ctx, "k_histogram");
-    k_bin_offsets<kBits><<<passes, R, 0, ctx->stream>>>(hist);
-    FL_CHECK_LAUNCH(ctx, "k_bin_offsets");
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)tiles);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
     uint64_t* ks[2] = {keys, kalt};
     uint32_t* vs[2] = {vals, valt};
     int cur = 0;
@@ -315,9 +342,11 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
         uint32_t* status = (uint32_t*)(stat0 + ps * stat_stride);
         unsigned* ticket = (unsigned*)(status + tiles * R);
         int sh = begin_bit + kBits * ps;
-        k_onesweep<kThreads, kBits, kItems><<<(unsigned)tiles, kThreads, smem, ctx->stream>>>(
-            ks[cur], vs[cur], ks[cur ^ 1], vs[cur ^ 1], n, sh, digit_mask(end_bit, sh, kBits), hist + ps * R, status,
-            ticket, ctx->dev_status);
+        const uint64_t* kin = ks[cur];
+        const uint32_t* vin = vs[cur];
+        const uint32_t* offs = hist + ps * R;
+        cudaLaunchKernelEx(&cfg, k_onesweep<kThreads, kBits, kItems>, kin, vin, ks[cur ^ 1], vs[cur ^ 1], n, sh,
+                           digit_mask(end_bit, sh, kBits), offs, status, ticket, ctx->dev_status);
         FL_CHECK_LAUNCH(ctx, "k_onesweep");
         cur ^= 1;
     }

@@ -10,7 +10,7 @@ from fluidloom_gb300 import DeviceArray
 
 pytestmark = pytest.mark.gpu
 
-SMALL = 1 << 19  # the most keys a small-tile sort takes
+SMALL = 1 << 20  # the most keys a small-tile sort takes
 
 
 @pytest.mark.parametrize("shape", [(8, 256), (8, 512), (9, 256), (9, 512)])
