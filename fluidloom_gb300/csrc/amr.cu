@@ -116,8 +116,8 @@ __global__ void k_shadow_update(fl_mesh_dev m, int mode, int max_level, uint8_t*
 // each on six of them, so that a leaf's lookups -- a key encoding and a random table slot per level
 // tried -- overlap instead of following one another (67,000 leaves: a thread a leaf 38 us, 20 now).
 __global__ void __launch_bounds__(kT) k_detect_face6(fl_mesh_dev m, fl_domain_dev dom, const uint64_t* __restrict__ tk,
-                                                     const uint32_t* __restrict__ tv, int lg,
-                                                     const uint8_t* __restrict__ shadow, uint8_t* __restrict__ viol,
+                                                     int lg, const uint8_t* __restrict__ shadow,
+                                                     uint8_t* __restrict__ viol,
                                                      uint32_t* __restrict__ count) {
     __shared__ KeyTables T;
     fl_keys_fill_tables(T.t1, T.t3, false);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kT) k_detect_face6(fl_mesh_dev m, fl_domain_de
             else if ((f >> 1) == 1) p[1] += move;
             else p[2] += move;
             if (fold3(p, d, dom.anchor_level)) {
-                const uint32_t r = fl_locate(T.t1, T.t3, tk, tv, lg, shadow, dom, cs, m.case_id != nullptr, p, sl);
+                const uint32_t r = fl_locate(T.t1, T.t3, tk, nullptr, lg, shadow, dom, cs, m.case_id != nullptr, p, sl);
                 hit = r != FL_INVALID_INDEX && (int)shadow[r] > sl + 1;
             }
         }
@@ -332,9 +332,14 @@ __device__ __forceinline__ uint32_t sibling_in_run(const fl_probe& P, const fl_m
 // the octet's level wherever in the cell it lies; only when that point is
 // not covered (a mesh that does not fill its domain) are the cell's other
 // probe points tried.  Same answer as the 98 probes, from 56 on a filled mesh.
+// With members the groups are filed at once, numbered in the order they are
+// found (*groups counts them; group_of holds FL_INVALID_INDEX before), which a
+// regrid, where only the emission reads the numbers, need not fix: 25 M cells
+// a scan and a second pass less (a regrid and neighbour rows 3,005 us, 2,897 now).
 __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom, fl_locator L, int min_level,
                                                 int check26, const uint8_t* __restrict__ shadow,
-                                                uint32_t* __restrict__ is_leader, uint32_t* __restrict__ group_of) {
+                                                uint32_t* __restrict__ is_leader, uint32_t* __restrict__ group_of,
+                                                uint32_t* __restrict__ members, uint32_t* __restrict__ groups) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
     __shared__ uint8_t surf[56];  // the outside cells k = ux + 4 uy + 16 uz of the 4^3 grid of child-sized cells
@@ -355,7 +360,7 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
         const size_t mine = base + lane;
         const bool cand = mine < m.n && merge_candidate(m, mine, min_level);
         if (mine < m.n && !cand) is_leader[mine] = 0u;
-        if (mine < m.n) group_of[mine] = FL_INVALID_INDEX;  // k_members fills in the groups
+        if (!members && mine < m.n) group_of[mine] = FL_INVALID_INDEX;  // k_members fills in the groups
         unsigned cm = __ballot_sync(0xFFFFFFFFu, cand);
         while (cm) {
             const int n4 = min(__popc(cm), 4);  // candidates of this round
@@ -433,7 +438,19 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
                 }
                 bad4 = __reduce_or_sync(0xFFFFFFFFu, bad4);
             }
-            if (have && (lane & 7) == 0) is_leader[i] = ((lead4 >> grp) & 1u) && !((bad4 >> grp) & 1u) ? 1u : 0u;
+            const unsigned good4 = lead4 & ~bad4;
+            if (have && (lane & 7) == 0) is_leader[i] = (good4 >> grp) & 1u;
+            if (members && good4) {
+                uint32_t g = 0;
+                if (lane == 0) g = atomicAdd(groups, (uint32_t)__popc(good4));
+                g = __shfl_sync(0xFFFFFFFFu, g, 0) + (uint32_t)__popc(good4 & ((1u << grp) - 1u));
+                if ((good4 >> grp) & 1u) {
+                    // a search finds sibling c in lane c, a run has them in key order
+                    const int c = P.L.ids ? lane & 7 : (m.x[j] & 1) | ((m.y[j] & 1) << 1) | ((m.z[j] & 1) << 2);
+                    members[(size_t)g * 8 + c] = j;
+                    group_of[j] = g;
+                }
+            }
         }
     }
 }
@@ -800,10 +817,9 @@ static size_t fl_balance_act_bytes(size_t n) { return fl_align256(n) + fl_align2
 
 size_t fl_adapt_scratch_bytes(size_t n, uint64_t cap) {
     size_t b = 0;
-    b += fl_align256(n * 8);                 // cell keys (FACE6's hash table)
-    b += fl_align256(cap * 16);              // 16-byte-slot table
+    b += fl_align256(cap * 16);              // FACE6's hash table, 16-byte slots
     b += 2 * fl_align256(n) + fl_balance_act_bytes(n);  // shadow, viol, probing leaves
-    b += 4 * fl_align256(n * 4);             // leader, gid, group_of, cnt/off
+    b += 3 * fl_align256(n * 4);             // leader, group_of, cnt/off
     b += fl_align256(n * 4);                 // members (n/8 groups * 8)
     b += fl_align256(64);                    // counters
     b += fl_scan_scratch_bytes(n) + fl_align256(fl_locator_scratch_bytes(n)) + 4096;
@@ -826,7 +842,7 @@ size_t fl_adapt_scratch_bytes(size_t n, uint64_t cap) {
 // round only a leaf that will split can find one: only those probe (through the
 // list, like the later rounds).
 int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_dev& dom, const uint64_t* tk,
-                   const uint32_t* tv, uint64_t cap, const fl_locator* L, int mode, int max_level, int max_iters,
+                   uint64_t cap, const fl_locator* L, int mode, int max_level, int max_iters,
                    uint8_t* shadow, uint8_t* viol, uint8_t* act, uint32_t* counters, fl_balance_result* res,
                    bool balanced_input) {
     fl_balance_result r{};
@@ -849,7 +865,7 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
         uint32_t* list = (act && mode == 1 && (it > 0 || first_listed)) ? (uint32_t*)(act + fl_align256(md.n)) : nullptr;
         uint32_t* list_n = counters + 4;  // free until the merge grouping after balance
         if (mode == 0) {
-            k_detect_face6<<<fl_blocks(md.n * 8, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(md, dom, tk, tv, lg, shadow, viol,
+            k_detect_face6<<<fl_blocks(md.n * 8, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(md, dom, tk, lg, shadow, viol,
                                                                                        counters);
         } else {
             k_clear_u8<<<nb, kT, 0, ctx->stream>>>(viol, md.n);
@@ -887,9 +903,9 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
 // Scratch layout of one regrid (carved identically by both phases).
 struct AdaptWork {
     uint64_t cap;
-    uint64_t* keys; uint64_t* tk; uint32_t* tv;
+    uint64_t* tk;  // FACE6's table, 16-byte slots
     uint8_t* shadow; uint8_t* viol; uint8_t* act;
-    uint32_t* leader; uint32_t* gid; uint32_t* group_of; uint32_t* cnt; uint32_t* members; uint32_t* counters;
+    uint32_t* leader; uint32_t* group_of; uint32_t* cnt; uint32_t* members; uint32_t* counters;
     void* scan_scratch;
     void* locator;  // fl_locator_build scratch
 };
@@ -898,14 +914,11 @@ static AdaptWork carve_adapt(void* scratch, size_t n, bool with_case) {
     AdaptWork w;
     w.cap = fl_table_capacity(n);
     Carver cv{(char*)scratch};
-    w.keys = cv.take<uint64_t>(n);
     w.tk = cv.take<uint64_t>(2 * w.cap);
-    w.tv = nullptr;  // 16-byte slots
     w.shadow = cv.take<uint8_t>(n);
     w.viol = cv.take<uint8_t>(n);
     w.act = cv.take<uint8_t>(fl_balance_act_bytes(n));
     w.leader = cv.take<uint32_t>(n);
-    w.gid = cv.take<uint32_t>(n);
     w.group_of = cv.take<uint32_t>(n);
     w.cnt = cv.take<uint32_t>(n);
     w.members = cv.take<uint32_t>(n + 8);
@@ -934,15 +947,12 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
     if (rc) return rc;
     *order = L.ids;
     if (run_balance && cfg->balance_mode == 0) {
-        rc = fl_launch_cell_keys(ctx, mesh->x, mesh->y, mesh->z, mesh->level, mesh->case_id, dom.depth,
-                                 dom.anchor_level, w.keys, n);
-        if (rc) return rc;
-        rc = fl_hash_build_with(ctx, w.tk, w.tv, w.cap, w.keys, nullptr, n, mesh->level);  // level | index
+        rc = fl_hash_build_cells(ctx, w.tk, w.cap, md, dom);
         if (rc) return rc;
     }
     FL_TRY_CUDA(ctx, cudaMemsetAsync(w.counters, 0, 64, ctx->stream), "adapt counters");
     if (run_balance) {
-        rc = fl_balance_run(ctx, md, mesh->flags, dom, w.tk, w.tv, w.cap, &L, cfg->balance_mode,
+        rc = fl_balance_run(ctx, md, mesh->flags, dom, w.tk, w.cap, &L, cfg->balance_mode,
                             cfg->max_refinement_level, (int)cfg->max_balance_iterations, w.shadow, w.viol, w.act,
                             w.counters + 8, &s.balance, cfg->input_balanced != 0);
         if (rc) return rc;
@@ -956,12 +966,10 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
         FL_CHECK_LAUNCH(ctx, "k_shadow_update");
     }
     const unsigned wb = fl_blocks((n + 31) / 32 * 32, kT, ctx->num_sms * 8);  // a warp per 32 cells
-    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, check26, w.shadow, w.leader, w.group_of);
+    FL_TRY_CUDA(ctx, cudaMemsetAsync(w.group_of, 0xFF, n * 4, ctx->stream), "adapt groups");
+    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, check26, w.shadow, w.leader, w.group_of,
+                                          w.members, w.counters + 2);
     FL_CHECK_LAUNCH(ctx, "k_leaders");
-    rc = fl_scan_u32_with(ctx, w.leader, w.gid, n, w.counters + 2, w.scan_scratch);
-    if (rc) return rc;
-    k_members<<<wb, kT, 0, ctx->stream>>>(md, dom, L, w.leader, w.gid, w.members, w.group_of);
-    FL_CHECK_LAUNCH(ctx, "k_members");
     k_counts<<<nb, kT, 0, ctx->stream>>>(md, cfg->max_refinement_level, L.ids, w.leader, w.group_of, w.cnt, w.counters);
     FL_CHECK_LAUNCH(ctx, "k_counts");
     rc = fl_scan_u32_with(ctx, w.cnt, w.cnt, n, w.counters + 3, w.scan_scratch);
@@ -1051,16 +1059,14 @@ int fl_balance_enforce(fl_ctx* ctx, fl_mesh* mesh, const fl_adapt_config* cfg, f
     if (n == 0) { if (res) res->converged = 1; return FL_OK; }
     const bool face6 = cfg->balance_mode == 0;  // FACE6 probes shadow levels through the hash table
     uint64_t cap = face6 ? fl_table_capacity(n) : 0;
-    size_t need = fl_align256(n * 8) + fl_align256(cap * 16) + 2 * fl_align256(n) +
+    size_t need = fl_align256(cap * 16) + 2 * fl_align256(n) +
                   fl_balance_act_bytes(n) + 512 + 256 +
                   (face6 ? 0 : fl_locator_scratch_bytes(n));
     int rc = fl_scratch_reserve(ctx, need);
     if (rc) return rc;
     Carver cv{(char*)ctx->scratch};
     void* dcase = cv.take<char>(256);
-    uint64_t* keys = cv.take<uint64_t>(n);
-    uint64_t* tk = cv.take<uint64_t>(2 * cap);
-    uint32_t* tv = nullptr;  // 16-byte slots
+    uint64_t* tk = cv.take<uint64_t>(2 * cap);  // 16-byte slots
     uint8_t* shadow = cv.take<uint8_t>(n);
     uint8_t* viol = cv.take<uint8_t>(n);
     uint8_t* act = cv.take<uint8_t>(fl_balance_act_bytes(n));
@@ -1069,16 +1075,13 @@ int fl_balance_enforce(fl_ctx* ctx, fl_mesh* mesh, const fl_adapt_config* cfg, f
     fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material, mesh->case_id, n};
     fl_locator L{};
     if (face6) {
-        rc = fl_launch_cell_keys(ctx, mesh->x, mesh->y, mesh->z, mesh->level, mesh->case_id, dom.depth,
-                                 dom.anchor_level, keys, n);
-        if (rc) return rc;
-        rc = fl_hash_build_with(ctx, tk, tv, cap, keys, nullptr, n, mesh->level);
+        rc = fl_hash_build_cells(ctx, tk, cap, md, dom);
     } else {
         rc = fl_locator_build(ctx, md, dom, cv.p, &L);
     }
     if (rc) return rc;
     fl_balance_result r;
-    rc = fl_balance_run(ctx, md, mesh->flags, dom, tk, tv, cap, &L, cfg->balance_mode, cfg->max_refinement_level,
+    rc = fl_balance_run(ctx, md, mesh->flags, dom, tk, cap, &L, cfg->balance_mode, cfg->max_refinement_level,
                         (int)cfg->max_balance_iterations, shadow, viol, act, counters, &r, cfg->input_balanced != 0);
     if (rc) return rc;
     rc = fl_collect_device_status(ctx, "fl_balance_enforce");
@@ -1239,7 +1242,8 @@ int fl_merge(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg, const
     rc = fl_locator_build(ctx, md, dom, loc, &L, -1, false, false);
     if (rc) return rc;
     const unsigned wb = fl_blocks((n + 31) / 32 * 32, kT, ctx->num_sms * 8);  // a warp per 32 cells
-    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, 0, nullptr, leader, group_of);
+    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, 0, nullptr, leader, group_of, nullptr,
+                                          nullptr);
     FL_CHECK_LAUNCH(ctx, "k_leaders");
     rc = fl_scan_u32_with(ctx, leader, gid, n, total, ss);
     if (rc) return rc;

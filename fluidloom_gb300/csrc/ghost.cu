@@ -225,19 +225,13 @@ int fl_interp_trilinear(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config*
     if (mesh->case_id) return fl_set_error(ctx, FL_E_INVALID_ARG, "fl_interp_trilinear: single-case meshes only");
     size_t n = mesh->num_cells;
     uint64_t cap = fl_table_capacity(n ? n : 1);
-    int rc = fl_scratch_reserve(ctx, 256 + fl_align256(n * 8 + 8) + fl_align256(cap * 16));
+    int rc = fl_scratch_reserve(ctx, 256 + fl_align256(cap * 16));
     if (rc) return rc;
-    char* p = (char*)ctx->scratch;
-    void* dcase = p; p += 256;
-    uint64_t* keys = (uint64_t*)p; p += fl_align256(n * 8 + 8);
-    uint64_t* tk = (uint64_t*)p;
+    void* dcase = ctx->scratch;
+    uint64_t* tk = (uint64_t*)((char*)ctx->scratch + 256);
     fl_domain_dev dom = fl_domain_from_config(ctx, cfg, dcase);
-    if (n) {
-        rc = fl_launch_cell_keys(ctx, mesh->x, mesh->y, mesh->z, mesh->level, nullptr, dom.depth, dom.anchor_level,
-                                 keys, n);
-        if (rc) return rc;
-    }
-    rc = fl_hash_build_with(ctx, tk, nullptr, cap, keys, nullptr, n, mesh->level);
+    fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material, nullptr, n};
+    rc = fl_hash_build_cells(ctx, tk, cap, md, dom);
     if (rc) return rc;
     k_interp<<<fl_blocks((nq + 3) / 4 * 32, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
         dom, tk, fl_hash_lg(cap), field, C, fx, fy, fz, flevel, nq, out);

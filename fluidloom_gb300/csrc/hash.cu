@@ -34,34 +34,17 @@ __global__ void k_hash_clear(uint64_t* __restrict__ tk, uint32_t* __restrict__ t
     }
 }
 
-// The value input i stores: vals[i], or (level << kPackedIdxBits) | i, or i.
-__device__ __forceinline__ uint32_t hash_value_of(size_t i, const uint32_t* __restrict__ vals,
-                                                  const uint8_t* __restrict__ levels) {
-    if (vals) return vals[i];
-    if (levels) return ((uint32_t)levels[i] << kPackedIdxBits) | (uint32_t)i;
-    return (uint32_t)i;
-}
-
-// Insertion into the 16-byte-slot layout: the slot's key word by CAS, its value word by a 64-bit
-// maximum of (input index + 1) << 32 | value, so a repeated key ends with the value of its last
-// input whatever the order of the threads.
-__device__ __forceinline__ void hash_store_max(uint64_t* tk, uint64_t s, size_t i, uint32_t v) {
-    atomicMax((unsigned long long*)(tk + 2 * s + 1), ((unsigned long long)(i + 1) << 32) | v);
-}
-
-// Insertion into separate key and value arrays: the thread whose CAS claims an empty slot stores
-// its value with a plain store; a thread that finds its key already there flags the build
-// (FL_DEVSTAT_HASH_DUPS) and stores nothing.  Without repeated keys that is the table; with them
-// the three passes below give each repeated key the value of its last input.
-template <bool kPacked>
+// Insertion: the thread whose CAS claims an empty slot stores its value with a
+// plain store; a thread that finds its key already there flags the build
+// (FL_DEVSTAT_HASH_DUPS) and stores nothing.  Without repeated keys that is
+// the table; with them the passes below give each repeated key the value
+// of its last input.
 __global__ void __launch_bounds__(256) k_hash_insert(uint64_t* __restrict__ tk, uint32_t* __restrict__ tv, int lg,
                                                      const uint64_t* __restrict__ keys,
-                                                     const uint32_t* __restrict__ vals,
-                                                     const uint8_t* __restrict__ levels, size_t n,
+                                                     const uint32_t* __restrict__ vals, size_t n,
                                                      uint32_t* dev_status) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const uint64_t mask = (1ull << lg) - 1;
-    constexpr int sw = kPacked ? 2 : 1;
     bool dup = false;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const uint64_t k = keys[i];
@@ -69,18 +52,48 @@ __global__ void __launch_bounds__(256) k_hash_insert(uint64_t* __restrict__ tk, 
         uint64_t s = fl_hash_slot(k, lg);
         int p = 0;
         for (; p < kProbeLimit; ++p) {
-            const unsigned long long prev = atomicCAS((unsigned long long*)(tk + s * sw), FL_EMPTY_KEY, k);
+            const unsigned long long prev = atomicCAS((unsigned long long*)(tk + s), FL_EMPTY_KEY, k);
+            if (prev == FL_EMPTY_KEY) tv[s] = vals ? vals[i] : (uint32_t)i;
+            if (prev == k) dup = true;
+            if (prev == FL_EMPTY_KEY || prev == k) break;
+            s = (s + 1) & mask;
+        }
+        if (p == kProbeLimit) atomicAdd(dev_status + FL_DEVSTAT_HASH_OVERFLOW, 1u);
+    }
+    if (dup) atomicOr(dev_status + FL_DEVSTAT_HASH_DUPS, 1u);
+}
+
+// A mesh's cells under their anchor keys (k_cell_keys') in the 16-byte-slot layout: the key worked out
+// on the way in, the slot's key word by CAS, its value word by a 64-bit maximum of (cell + 1) << 32 |
+// level << 27 | cell, so that of cells with one key the last is kept whatever the order of the threads.
+// Keys and table in one pass (262,144 cells, ghosts filled from them: 80 us with k_cell_keys before, 74 now).
+__global__ void __launch_bounds__(256) k_hash_insert_cells(uint64_t* __restrict__ tk, int lg, fl_mesh_dev m,
+                                                           fl_domain_dev dom, uint32_t* dev_status) {
+    __shared__ __align__(16) uint8_t t1[96];
+    __shared__ __align__(16) uint16_t t3c[12 * 512];
+    fl_keys_fill_tables_cat(t1, t3c);
+    __syncthreads();
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const uint64_t mask = (1ull << lg) - 1;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m.n; i += stride) {
+        const int l = m.level[i], sh = dom.anchor_level - l;
+        uint64_t k = fl_hilbert_encode_cat(t1, t3c, (uint32_t)m.x[i] << sh, (uint32_t)m.y[i] << sh,
+                                           (uint32_t)m.z[i] << sh, dom.depth);
+        if (m.case_id) k |= (uint64_t)m.case_id[i] << (3 * dom.depth);
+        if (k == FL_EMPTY_KEY) continue;
+        uint64_t s = fl_hash_slot(k, lg);
+        int p = 0;
+        for (; p < kProbeLimit; ++p) {
+            const unsigned long long prev = atomicCAS((unsigned long long*)(tk + 2 * s), FL_EMPTY_KEY, k);
             if (prev == FL_EMPTY_KEY || prev == k) {
-                if (kPacked) hash_store_max(tk, s, i, hash_value_of(i, vals, levels));
-                else if (prev == FL_EMPTY_KEY) tv[s] = hash_value_of(i, vals, levels);
-                else dup = true;
+                atomicMax((unsigned long long*)(tk + 2 * s + 1),
+                          ((unsigned long long)(i + 1) << 32) | ((uint32_t)l << kPackedIdxBits) | (uint32_t)i);
                 break;
             }
             s = (s + 1) & mask;
         }
         if (p == kProbeLimit) atomicAdd(dev_status + FL_DEVSTAT_HASH_OVERFLOW, 1u);
     }
-    if (!kPacked && dup) atomicOr(dev_status + FL_DEVSTAT_HASH_DUPS, 1u);
 }
 
 // Repeated keys only, launched when a build into separate arrays met some (three launches that
@@ -111,7 +124,7 @@ __global__ void k_hash_dup_values(uint32_t* __restrict__ tv, const uint32_t* __r
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += stride) {
         const uint32_t w = win[i];
-        if (w) tv[i] = hash_value_of(w - 1, vals, nullptr);
+        if (w) tv[i] = vals ? vals[w - 1] : w - 1;
     }
 }
 
@@ -756,20 +769,14 @@ int fl_hash_lg(uint64_t cap) {
     return lg;
 }
 
-int fl_hash_build_with(fl_ctx* ctx, uint64_t* tk, uint32_t* tv, uint64_t cap, const uint64_t* keys,
-                       const uint32_t* vals, size_t n, const uint8_t* levels) {
-    if (levels && !vals && n >= ((size_t)1 << kPackedIdxBits))
-        return fl_set_error(ctx, FL_E_CAPACITY, "a mesh of 2^27 or more cells");
-    unsigned cb = fl_blocks(cap, 256, ctx->num_sms * 8);
-    k_hash_clear<<<cb, 256, 0, ctx->stream>>>(tk, tv, cap);
+int fl_hash_build_cells(fl_ctx* ctx, uint64_t* tk, uint64_t cap, const fl_mesh_dev& m, const fl_domain_dev& dom) {
+    if (m.n >= ((size_t)1 << kPackedIdxBits)) return fl_set_error(ctx, FL_E_CAPACITY, "a mesh of 2^27 or more cells");
+    k_hash_clear<<<fl_blocks(cap, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(tk, nullptr, cap);
     FL_CHECK_LAUNCH(ctx, "k_hash_clear");
-    if (n == 0) return FL_OK;
-    const uint8_t* lv = vals ? nullptr : levels;
-    int lg = fl_hash_lg(cap);
-    unsigned nb = fl_blocks(n, 256, ctx->num_sms * 8);
-    if (tv) k_hash_insert<false><<<nb, 256, 0, ctx->stream>>>(tk, tv, lg, keys, vals, lv, n, ctx->dev_status);
-    else k_hash_insert<true><<<nb, 256, 0, ctx->stream>>>(tk, nullptr, lg, keys, vals, lv, n, ctx->dev_status);
-    FL_CHECK_LAUNCH(ctx, "k_hash_insert");
+    if (m.n == 0) return FL_OK;
+    k_hash_insert_cells<<<fl_blocks(m.n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(tk, fl_hash_lg(cap), m, dom,
+                                                                                       ctx->dev_status);
+    FL_CHECK_LAUNCH(ctx, "k_hash_insert_cells");
     return FL_OK;
 }
 
@@ -798,9 +805,14 @@ int fl_hash_build(fl_ctx* ctx, uint64_t* table_keys, uint32_t* table_vals, uint6
         return fl_set_error(ctx, FL_E_INVALID_ARG, "fl_hash_build: bad table or capacity not a power of two");
     if (n > capacity) return fl_set_error(ctx, FL_E_CAPACITY, "fl_hash_build: more keys than slots");
     FL_TRY_CUDA(ctx, cudaMemsetAsync(ctx->dev_status + FL_DEVSTAT_HASH_DUPS, 0, 4, ctx->stream), "hash flag");
-    int rc = fl_hash_build_with(ctx, table_keys, table_vals, capacity, keys, vals, n);
-    if (rc) return rc;
-    rc = fl_collect_device_status(ctx, "fl_hash_build");
+    k_hash_clear<<<fl_blocks(capacity, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(table_keys, table_vals, capacity);
+    FL_CHECK_LAUNCH(ctx, "k_hash_clear");
+    if (n) {
+        k_hash_insert<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+            table_keys, table_vals, fl_hash_lg(capacity), keys, vals, n, ctx->dev_status);
+        FL_CHECK_LAUNCH(ctx, "k_hash_insert");
+    }
+    int rc = fl_collect_device_status(ctx, "fl_hash_build");
     if (rc || !ctx->host_status[FL_DEVSTAT_HASH_DUPS]) return rc;
     // repeated keys: the winner of each slot in a second round
     rc = fl_scratch_reserve(ctx, capacity * 4);

@@ -242,10 +242,6 @@ int fl_neighbours_octree(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev&
 
 int fl_hash_lg(uint64_t cap);
 uint64_t fl_table_capacity(size_t n);
-// Clear + build; tv == nullptr builds the 16-byte-slot layout in tk (2 * cap
-// words; a repeated key keeps the value of its last input), else the API's
-// arrays, where a build that met repeated keys sets FL_DEVSTAT_HASH_DUPS and
-// leaves them to the caller.  With `levels` (and no vals) the values are
-// levels[i] << 27 | i (n < 2^27, else FL_E_CAPACITY).
-int fl_hash_build_with(fl_ctx* ctx, uint64_t* tk, uint32_t* tv, uint64_t cap, const uint64_t* keys,
-                       const uint32_t* vals, size_t n, const uint8_t* levels = nullptr);
+// Clear + build of the 16-byte-slot table over a mesh's cells (tk: 2 * cap words): anchor key ->
+// level << 27 | cell, of cells with one key the last.  n < 2^27, else FL_E_CAPACITY.
+int fl_hash_build_cells(fl_ctx* ctx, uint64_t* tk, uint64_t cap, const fl_mesh_dev& m, const fl_domain_dev& dom);
