@@ -75,11 +75,32 @@ __device__ __forceinline__ uint8_t shadow_of(const fl_mesh_dev& m, size_t i, int
 
 // Shadow levels; lowest[0] / lowest[1] (when given) receive their minimum and
 // maximum; refining (when given) a byte per leaf, set where the leaf will split.
+// FULL26 takes four leaves a thread where the columns' addresses allow it (25 M
+// leaves, 7 bytes each: 73 us, 40 now).
 __global__ void k_shadow(fl_mesh_dev m, int mode, int max_level, uint8_t* __restrict__ shadow,
                          uint32_t* __restrict__ lowest, uint8_t* __restrict__ refining) {
     size_t stride = (size_t)gridDim.x * blockDim.x;
     unsigned lo = 255u, hi = 0u;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m.n; i += stride) {
+    const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool quads = mode == 1 && ((uintptr_t)m.flags & 15) == 0 &&
+                       (((uintptr_t)m.level | (uintptr_t)m.state | (uintptr_t)shadow | (uintptr_t)refining) & 3) == 0;
+    const size_t nq = quads ? m.n / 4 : 0;
+    for (size_t q = t0; q < nq; q += stride) {
+        const int4 f = ((const int4*)m.flags)[q];
+        const uint32_t lv = ((const uint32_t*)m.level)[q], st = ((const uint32_t*)m.state)[q];
+        const int fl[4] = {f.x, f.y, f.z, f.w};
+        uint32_t up = 0;
+        for (int k = 0; k < 4; ++k) {
+            const unsigned l = (lv >> (8 * k)) & 255u;
+            const unsigned u = fl[k] > 0 && ((st >> (8 * k)) & 255u) == 0 && (int)l < max_level ? 1u : 0u;
+            up |= u << (8 * k);
+            lo = min(lo, l + u);
+            hi = max(hi, l + u);
+        }
+        ((uint32_t*)shadow)[q] = lv + up;  // no carry: a leaf above max_level - 1 is not raised
+        if (refining) ((uint32_t*)refining)[q] = up;
+    }
+    for (size_t i = 4 * nq + t0; i < m.n; i += stride) {
         const uint8_t v = mode == 0 ? m.level[i] : shadow_of(m, i, mode, max_level);
         shadow[i] = v;
         if (refining) refining[i] = v > m.level[i] ? 1 : 0;
@@ -332,10 +353,15 @@ __device__ __forceinline__ uint32_t sibling_in_run(const fl_probe& P, const fl_m
 // the octet's level wherever in the cell it lies; only when that point is
 // not covered (a mesh that does not fill its domain) are the cell's other
 // probe points tried.  Same answer as the 98 probes, from 56 on a filled mesh.
-// With members the groups are filed at once, numbered in the order they are
+// With members the groups are filed at once, the leader's entry of group_of
+// marked by kLeads instead of a word in is_leader, numbered in the order they are
 // found (*groups counts them; group_of holds FL_INVALID_INDEX before), which a
 // regrid, where only the emission reads the numbers, need not fix: 25 M cells
 // a scan and a second pass less (a regrid and neighbour rows 3,005 us, 2,897 now).
+// In group_of, a leader's group (there are at most n / 8 < 2^29) -- so the entries with the top bit, the
+// leaders' and FL_INVALID_INDEX of the cells in no group, are those of the cells that make a new one.
+constexpr uint32_t kLeads = 0x80000000u;
+
 __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom, fl_locator L, int min_level,
                                                 int check26, const uint8_t* __restrict__ shadow,
                                                 uint32_t* __restrict__ is_leader, uint32_t* __restrict__ group_of,
@@ -359,8 +385,10 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
          base += warps * 32) {
         const size_t mine = base + lane;
         const bool cand = mine < m.n && merge_candidate(m, mine, min_level);
-        if (mine < m.n && !cand) is_leader[mine] = 0u;
-        if (!members && mine < m.n) group_of[mine] = FL_INVALID_INDEX;  // k_members fills in the groups
+        if (!members && mine < m.n) {  // k_members fills in the groups
+            if (!cand) is_leader[mine] = 0u;
+            group_of[mine] = FL_INVALID_INDEX;
+        }
         unsigned cm = __ballot_sync(0xFFFFFFFFu, cand);
         while (cm) {
             const int n4 = min(__popc(cm), 4);  // candidates of this round
@@ -439,7 +467,7 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
                 bad4 = __reduce_or_sync(0xFFFFFFFFu, bad4);
             }
             const unsigned good4 = lead4 & ~bad4;
-            if (have && (lane & 7) == 0) is_leader[i] = (good4 >> grp) & 1u;
+            if (!members && have && (lane & 7) == 0) is_leader[i] = (good4 >> grp) & 1u;
             if (members && good4) {
                 uint32_t g = 0;
                 if (lane == 0) g = atomicAdd(groups, (uint32_t)__popc(good4));
@@ -448,7 +476,7 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
                     // a search finds sibling c in lane c, a run has them in key order
                     const int c = P.L.ids ? lane & 7 : (m.x[j] & 1) | ((m.y[j] & 1) << 1) | ((m.z[j] & 1) << 2);
                     members[(size_t)g * 8 + c] = j;
-                    group_of[j] = g;
+                    group_of[j] = c ? g : g | kLeads;
                 }
             }
         }
@@ -459,7 +487,7 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
 // at a time (lane 8s + c: sibling c of the s-th).
 __global__ void __launch_bounds__(kT) k_members(fl_mesh_dev m, fl_domain_dev dom, fl_locator L,
                                                 const uint32_t* __restrict__ is_leader,
-                                                const uint32_t* __restrict__ gid, uint32_t* __restrict__ members,
+                                                   const uint32_t* __restrict__ gid, uint32_t* __restrict__ members,
                                                 uint32_t* __restrict__ group_of) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
@@ -501,7 +529,6 @@ __global__ void __launch_bounds__(kT) k_members(fl_mesh_dev m, fl_domain_dev dom
 // t-th, or t when order is null), and the split and surviving cells counted
 // (counters[4], [5]; one atomic each per block).
 __global__ void __launch_bounds__(kT) k_counts(fl_mesh_dev m, int max_level, const uint32_t* __restrict__ order,
-                                               const uint32_t* __restrict__ is_leader,
                                                const uint32_t* __restrict__ group_of, uint32_t* __restrict__ cnt,
                                                uint32_t* __restrict__ counters) {
     __shared__ uint32_t s_sum[2];
@@ -512,10 +539,11 @@ __global__ void __launch_bounds__(kT) k_counts(fl_mesh_dev m, int max_level, con
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < m.n; t += stride) {
         const size_t i = order ? order[t] : t;
         const bool split = m.flags[i] > 0 && m.state[i] == 0 && m.level[i] < max_level;
-        const bool grouped = group_of[i] != FL_INVALID_INDEX;
+        const uint32_t g = group_of[i];
+        const bool grouped = g != FL_INVALID_INDEX;
         ns += split ? 1u : 0u;
         nv += !split && !grouped ? 1u : 0u;
-        cnt[t] = split ? 8u : (grouped ? (is_leader[i] ? 1u : 0u) : 1u);
+        cnt[t] = split ? 8u : g >> 31;
     }
     ns = __reduce_add_sync(0xFFFFFFFFu, ns);
     nv = __reduce_add_sync(0xFFFFFFFFu, nv);
@@ -559,10 +587,9 @@ __device__ __forceinline__ void emit_row(int kind, size_t i, uint32_t j, uint32_
 // neighbouring ones, so a cell's columns are loaded together and go straight
 // out.  The other groups go into list for k_emit.  25 M cells of which a few
 // per cent change: 492 us for all groups in k_emit (64 registers, three
-// dependent loads a cell), 161 for both.
+// dependent loads a cell), 177 for both.
 __global__ void __launch_bounds__(kT, 8) k_emit_plain(fl_mesh_dev m, int max_level, const uint32_t* __restrict__ order,
                                                       const uint32_t* __restrict__ off,
-                                                      const uint32_t* __restrict__ is_leader,
                                                       const uint32_t* __restrict__ group_of,
                                                       const uint32_t* __restrict__ members, fl_mesh_out out,
                                                       uint32_t* __restrict__ osrc, uint8_t* __restrict__ okind,
@@ -577,13 +604,12 @@ __global__ void __launch_bounds__(kT, 8) k_emit_plain(fl_mesh_dev m, int max_lev
         const int32_t x = m.x[i], y = m.y[i], z = m.z[i], fl = m.flags[i];
         const int l = m.level[i];
         const uint8_t state = m.state[i];
-        const uint32_t material = m.material[i], g = group_of[i], o = in ? off[t] : 0u;
+        const uint32_t material = m.material[i], gl = group_of[i], o = in ? off[t] : 0u;
         if (__any_sync(0xFFFFFFFFu, in && fl > 0 && state == 0 && l < max_level)) {
             if (lane == 0) list[atomicAdd(list_n, 1u)] = (uint32_t)(t0 >> 5);
             continue;
         }
-        const bool grouped = g != FL_INVALID_INDEX;
-        const bool makes = in && (!grouped || is_leader[i]);
+        const bool grouped = gl != FL_INVALID_INDEX, makes = in && gl >= kLeads;
         if (makes) {
             const int up = grouped ? 1 : 0;
             out.x[o] = x >> up;
@@ -594,7 +620,7 @@ __global__ void __launch_bounds__(kT, 8) k_emit_plain(fl_mesh_dev m, int max_lev
             out.material[o] = material;
             out.flags[o] = 0;
             if (out.case_id) out.case_id[o] = m.case_id ? m.case_id[i] : 0;
-            if (osrc) osrc[o] = up ? g : (uint32_t)i;
+            if (osrc) osrc[o] = up ? gl & ~kLeads : (uint32_t)i;
             if (okind) okind[o] = up ? 9 : 8;
         }
         if (fin && C) {
@@ -603,7 +629,7 @@ __global__ void __launch_bounds__(kT, 8) k_emit_plain(fl_mesh_dev m, int max_lev
                 float* fo = fout + (size_t)__shfl_sync(0xFFFFFFFFu, o, 0) * C;
                 for (uint32_t e = lane; e < 32u * C; e += 32u) fo[e] = sp[e];
             } else if (makes) {
-                emit_row(grouped ? 2 : 3, i, o, g, members, fin, fout, C, rule);
+                emit_row(grouped ? 2 : 3, i, o, gl & ~kLeads, members, fin, fout, C, rule);
             }
         }
     }
@@ -612,7 +638,6 @@ __global__ void __launch_bounds__(kT, 8) k_emit_plain(fl_mesh_dev m, int max_lev
 // The groups with split cells: their new cells staged in shared memory, column by column.
 __global__ void __launch_bounds__(kT) k_emit(fl_mesh_dev m, fl_domain_dev dom, int max_level,
                                              const uint32_t* __restrict__ order, const uint32_t* __restrict__ off,
-                                             const uint32_t* __restrict__ is_leader,
                                              const uint32_t* __restrict__ group_of,
                                              const uint32_t* __restrict__ members, fl_mesh_out out,
                                              uint32_t* __restrict__ osrc, uint8_t* __restrict__ okind,
@@ -644,7 +669,8 @@ __global__ void __launch_bounds__(kT) k_emit(fl_mesh_dev m, fl_domain_dev dom, i
                 st = fl_hilbert_state_cat(t1, t3c, (uint32_t)m.x[i], (uint32_t)m.y[i], (uint32_t)m.z[i],
                                           dom.depth - dom.anchor_level + l);
             } else if ((g = group_of[i]) != FL_INVALID_INDEX) {
-                if (is_leader[i]) { kind = 2; cnt = 1; }
+                if (g >> 31) { kind = 2; cnt = 1; }
+                g &= ~kLeads;
             } else {
                 kind = 3;
                 cnt = 1;
@@ -819,7 +845,7 @@ size_t fl_adapt_scratch_bytes(size_t n, uint64_t cap) {
     size_t b = 0;
     b += fl_align256(cap * 16);              // FACE6's hash table, 16-byte slots
     b += 2 * fl_align256(n) + fl_balance_act_bytes(n);  // shadow, viol, probing leaves
-    b += 3 * fl_align256(n * 4);             // leader, group_of, cnt/off
+    b += 2 * fl_align256(n * 4);             // group_of, cnt/off
     b += fl_align256(n * 4);                 // members (n/8 groups * 8)
     b += fl_align256(64);                    // counters
     b += fl_scan_scratch_bytes(n) + fl_align256(fl_locator_scratch_bytes(n)) + 4096;
@@ -905,7 +931,7 @@ struct AdaptWork {
     uint64_t cap;
     uint64_t* tk;  // FACE6's table, 16-byte slots
     uint8_t* shadow; uint8_t* viol; uint8_t* act;
-    uint32_t* leader; uint32_t* group_of; uint32_t* cnt; uint32_t* members; uint32_t* counters;
+    uint32_t* group_of; uint32_t* cnt; uint32_t* members; uint32_t* counters;
     void* scan_scratch;
     void* locator;  // fl_locator_build scratch
 };
@@ -918,7 +944,6 @@ static AdaptWork carve_adapt(void* scratch, size_t n, bool with_case) {
     w.shadow = cv.take<uint8_t>(n);
     w.viol = cv.take<uint8_t>(n);
     w.act = cv.take<uint8_t>(fl_balance_act_bytes(n));
-    w.leader = cv.take<uint32_t>(n);
     w.group_of = cv.take<uint32_t>(n);
     w.cnt = cv.take<uint32_t>(n);
     w.members = cv.take<uint32_t>(n + 8);
@@ -967,10 +992,10 @@ int fl_adapt_prepare(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cf
     }
     const unsigned wb = fl_blocks((n + 31) / 32 * 32, kT, ctx->num_sms * 8);  // a warp per 32 cells
     FL_TRY_CUDA(ctx, cudaMemsetAsync(w.group_of, 0xFF, n * 4, ctx->stream), "adapt groups");
-    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, check26, w.shadow, w.leader, w.group_of,
-                                          w.members, w.counters + 2);
+    k_leaders<<<wb, kT, 0, ctx->stream>>>(md, dom, L, cfg->min_refinement_level, check26, w.shadow, nullptr,
+                                          w.group_of, w.members, w.counters + 2);
     FL_CHECK_LAUNCH(ctx, "k_leaders");
-    k_counts<<<nb, kT, 0, ctx->stream>>>(md, cfg->max_refinement_level, L.ids, w.leader, w.group_of, w.cnt, w.counters);
+    k_counts<<<nb, kT, 0, ctx->stream>>>(md, cfg->max_refinement_level, L.ids, w.group_of, w.cnt, w.counters);
     FL_CHECK_LAUNCH(ctx, "k_counts");
     rc = fl_scan_u32_with(ctx, w.cnt, w.cnt, n, w.counters + 3, w.scan_scratch);
     if (rc) return rc;
@@ -1005,11 +1030,11 @@ int fl_adapt_finish(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config* cfg
     uint32_t* list = (uint32_t*)w.viol;      // groups of 32 cells: n / 8 of the balance's n bytes
     uint32_t* list_n = w.counters + 6;       // still 0
     k_emit_plain<<<fl_blocks(n, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(
-        md, cfg->max_refinement_level, order, w.cnt, w.leader, w.group_of, w.members, o, osrc, okind, fields, out_fields,
+        md, cfg->max_refinement_level, order, w.cnt, w.group_of, w.members, o, osrc, okind, fields, out_fields,
         C, cfg->averaging_rule, list, list_n);
     FL_CHECK_LAUNCH(ctx, "k_emit_plain");
     k_emit<<<fl_blocks(n, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(
-        md, dom, cfg->max_refinement_level, order, w.cnt, w.leader, w.group_of, w.members, o, osrc, okind, fields,
+        md, dom, cfg->max_refinement_level, order, w.cnt, w.group_of, w.members, o, osrc, okind, fields,
         out_fields, C, cfg->averaging_rule, list, list_n);
     FL_CHECK_LAUNCH(ctx, "k_emit");
     if (omembers && num_groups)

@@ -170,37 +170,53 @@ __global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__
 // Run start of every leaf divided by 8^cut: the anchor shifted down by cut,
 // encoded at depth - cut levels, the low 3(A - l - cut) bits cleared (the case
 // id above bit 3 * (depth - cut)).
+//
+// unsorted (when given) is set when some run start is smaller than the one
+// before it.  A warp takes a range of consecutive leaves and keeps the last of
+// 32 for the next 32, so only the start of its range is encoded twice (25 M
+// leaves: 107 us and a pass of 41 over the keys, 135 now).
 __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev dom, int cut,
-                                                  const uint32_t* __restrict__ deepest, uint64_t* __restrict__ keys) {
+                                                  const uint32_t* __restrict__ deepest, uint64_t* __restrict__ keys,
+                                                  uint32_t* __restrict__ unsorted) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
     __syncthreads();
     if (cut < 0) cut = max(dom.anchor_level - (int)*deepest, 0);  // not known on the host yet
     const int dc = dom.depth - cut;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m.n; i += stride) {
+    auto key_of = [&](size_t i) {
         const int sh = dom.anchor_level - m.level[i];
         uint64_t k = fl_hilbert_encode_cat(t1, t3c, ((uint32_t)m.x[i] << sh) >> cut, ((uint32_t)m.y[i] << sh) >> cut,
                                            ((uint32_t)m.z[i] << sh) >> cut, dc);
         k &= ~((1ull << (3 * (sh - cut))) - 1);
         if (m.case_id) k |= (uint64_t)m.case_id[i] << (3 * dc);
-        keys[i] = k;
+        return k;
+    };
+    const int lane = threadIdx.x & 31;
+    const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5), pieces = (m.n + 31) / 32;
+    const size_t per = (pieces + warps - 1) / warps * 32;
+    const size_t first = ((size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per;
+    if (first >= m.n) return;
+    const size_t end = min(first + per, m.n);
+    uint64_t last = unsorted && first ? key_of(first - 1) : 0;
+    bool bad = false;
+    for (size_t i0 = first; i0 < end; i0 += 32) {
+        const size_t i = i0 + lane;
+        const uint64_t k = i < end ? key_of(i) : ~0ull;
+        if (i < end) keys[i] = k;
+        if (unsorted) {
+            uint64_t before = __shfl_up_sync(0xFFFFFFFFu, k, 1);
+            if (lane == 0) before = last;
+            bad = bad || k < before;
+            last = __shfl_sync(0xFFFFFFFFu, k, 31);
+        }
     }
+    if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) *unsorted = 1u;
 }
 
 __global__ void k_iota(uint32_t* __restrict__ ids, size_t n) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) ids[i] = (uint32_t)i;
-}
-
-// flag = 1 when some run start is smaller than the one before it.
-__global__ void k_check_sorted(const uint64_t* __restrict__ keys, size_t n, uint32_t* __restrict__ flag) {
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    bool bad = false;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += stride)
-        bad = bad || keys[i] < keys[i - 1];
-    if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1u;
 }
 
 // dir[b] = first run whose bucket is >= b, b in [0, nb]: run i fills the
@@ -637,12 +653,9 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
         FL_CHECK_LAUNCH(ctx, "k_level_range");
     }
     const int bound_cut = level_bound < 0 ? -1 : std::max(dom.anchor_level - level_bound, 0);
-    k_run_keys<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, dom, bound_cut, flag + 1, keys);
+    k_run_keys<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, dom, bound_cut, flag + 1, keys,
+                                                                                 in_key_order ? nullptr : flag);
     FL_CHECK_LAUNCH(ctx, "k_run_keys");
-    if (!in_key_order) {
-        k_check_sorted<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(keys, n, flag);
-        FL_CHECK_LAUNCH(ctx, "k_check_sorted");
-    }
     if (!in_key_order || level_bound < 0) {  // one wait for both
         const int rc = fl_read_back(ctx, hf, flag, level_bound < 0 ? 8 : 4, "locator");
         if (rc) return rc;
