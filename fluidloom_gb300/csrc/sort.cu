@@ -18,6 +18,7 @@
 // keys, or x 4 for up to kSmallSort keys (512: half the tiles and twice the
 // keys per digit run written, at 2 CTAs per SM; 256: 4 CTAs per SM with 8-bit
 // digits, 3 with 9-bit, whose threads then take two digits each).
+// Large sorts of many passes leave out low passes that the high ones decide (kPlannedSort).
 // Stable: ties keep input order, so (key, payload) pairs match std::stable_sort.
 #include "common.cuh"
 #include "scan.cuh"
@@ -41,12 +42,20 @@ __host__ __device__ constexpr uint32_t digit_mask(int end_bit, int sh, int bits)
     return end_bit - sh >= bits ? (1u << bits) - 1u : (1u << (end_bit - sh)) - 1u;
 }
 
+// A sort that may leave out passes keeps its state behind the histograms: the
+// histogram's block count, the low passes put off, whether they are needed.
+struct SortPlan {
+    unsigned done, defer, unsorted;
+};
+constexpr uint32_t kFewDigits = 32;
+
 // Every pass's histogram, then, in the block that finishes last (*done counts the
 // blocks, starting at 0), each pass's bins scanned in place to exclusive offsets: a
-// warp per pass, R / 32 consecutive bins a lane.
-template <int kBits>
+// warp per pass, R / 32 consecutive bins a lane.  With kPlanned it also puts off
+// the low passes that meet at most kFewDigits different digits.
+template <int kBits, bool kPlanned>
 __global__ void __launch_bounds__(256) k_histogram(const uint64_t* __restrict__ keys, size_t n, int begin_bit,
-                                                   int end_bit, int passes, uint32_t* hist, unsigned* done) {
+                                                   int end_bit, int passes, uint32_t* hist, SortPlan* plan) {
     constexpr int R = 1 << kBits;
     __shared__ uint32_t h[kMaxPasses][R];
     __shared__ bool last;
@@ -67,30 +76,47 @@ __global__ void __launch_bounds__(256) k_histogram(const uint64_t* __restrict__ 
     }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) last = atomicAdd(&plan->done, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
     const int lane = threadIdx.x & 31, p = threadIdx.x >> 5;  // 8 warps, at most 8 passes
-    if (p >= passes) return;
-    uint32_t* g = hist + p * R + lane * (R / 32);
-    uint32_t v[R / 32], sum = 0;
+    if (!kPlanned && p >= passes) return;
+    if (p < passes) {
+        uint32_t* g = hist + p * R + lane * (R / 32);
+        uint32_t v[R / 32], sum = 0;
 #pragma unroll
-    for (int j = 0; j < R / 32; ++j) {
-        v[j] = __ldcg(g + j);
-        sum += v[j];
+        for (int j = 0; j < R / 32; ++j) {
+            v[j] = __ldcg(g + j);
+            sum += v[j];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        uint32_t run = incl - sum;
+#pragma unroll
+        for (int j = 0; j < R / 32; ++j) {
+            g[j] = run;
+            run += v[j];
+        }
+        if (kPlanned) {
+            uint32_t used = 0;
+#pragma unroll
+            for (int j = 0; j < R / 32; ++j) used += v[j] ? 1u : 0u;
+            used = __reduce_add_sync(0xFFFFFFFFu, used);
+            if (lane == 0) h[p][0] = used;
+        }
     }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    uint32_t run = incl - sum;
-#pragma unroll
-    for (int j = 0; j < R / 32; ++j) {
-        g[j] = run;
-        run += v[j];
+    if (kPlanned) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int d = 0;
+            while (d < passes - 1 && h[d][0] <= kFewDigits) ++d;
+            plan->defer = (unsigned)d;
+        }
     }
 }
 
@@ -105,11 +131,16 @@ __host__ __device__ constexpr size_t onesweep_smem() {
            ((size_t)(kThreads / 32) * (1 << kBits) + 2 * (1 << kBits) + kThreads / 32) * 4;
 }
 
-template <int kThreads, int kBits, int kItems>
+// kMode 0: one pass from the first buffers into the second.  1: pass number `pass` of a sort that
+// may put passes off: nothing if this is one of them, else from the buffers where the passes run
+// before it left the pairs.  2: a pass put on after all (when the plan says so), by the blocks that
+// fit the GPU, a tile after another: most sorts need none of these, and so small a grid ends soonest.
+template <int kThreads, int kBits, int kItems, int kMode>
 __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 4 : 3))
-    k_onesweep(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
-               uint32_t* __restrict__ vout, size_t n, int shift, uint32_t dmask,
-               const uint32_t* __restrict__ bin_off, uint32_t* status, unsigned* ticket, uint32_t* dev_status) {
+    k_onesweep(uint64_t* __restrict__ first_k, uint32_t* __restrict__ first_v, uint64_t* __restrict__ second_k,
+               uint32_t* __restrict__ second_v, size_t n, int shift, uint32_t dmask,
+               const uint32_t* __restrict__ bin_off, uint32_t* status, unsigned* ticket, uint32_t* dev_status,
+               const SortPlan* plan, int pass, int passes) {
     constexpr int R = 1 << kBits;
     constexpr int kWarps = kThreads / 32;
     constexpr int kTile = kThreads * kItems;
@@ -126,14 +157,34 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
     __shared__ int s_tile;
     __shared__ int s_bad;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) { s_tile = (int)atomicAdd(ticket, 1u); s_bad = 0; }
-    for (int i = threadIdx.x; i < kWarps * R; i += kThreads) s_warp_hist[i] = 0;
+    if (kMode == 0) {
+        if (threadIdx.x == 0) { s_tile = (int)atomicAdd(ticket, 1u); s_bad = 0; }
+        for (int i = threadIdx.x; i < kWarps * R; i += kThreads) s_warp_hist[i] = 0;
+    }
     // the passes are launched programmatically: this much of a pass overlaps the one before it,
     // whose output is read from here on
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
+    bool swapped = false;
+    if (kMode != 0) {
+        // (every block waits above first: the pass after this one counts on the passes before)
+        const int defer = (int)ld_vol(&plan->defer);
+        if (kMode == 1 ? pass < defer : !ld_vol(&plan->unsorted)) return;
+        swapped = kMode == 1 ? (pass - defer) & 1 : (passes - defer + pass) & 1;
+    }
+    const uint64_t* __restrict__ kin = swapped ? second_k : first_k;
+    const uint32_t* __restrict__ vin = swapped ? second_v : first_v;
+    uint64_t* __restrict__ kout = swapped ? first_k : second_k;
+    uint32_t* __restrict__ vout = swapped ? first_v : second_v;
+    do {
+    if (kMode != 0) {
+        __syncthreads();
+        if (threadIdx.x == 0) { s_tile = (int)atomicAdd(ticket, 1u); s_bad = 0; }
+        for (int i = threadIdx.x; i < kWarps * R; i += kThreads) s_warp_hist[i] = 0;
+    }
     __syncthreads();
     const int tile = s_tile;
+    if (kMode == 2 && (size_t)tile * kTile >= n) return;
     const size_t tbase = (size_t)tile * kTile;
     const size_t wbase = tbase + (size_t)warp * 32 * kItems;
     const unsigned lt = (1u << lane) - 1u;
@@ -279,6 +330,40 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
         kout[pos] = kk;
         vout[pos] = s_vals[i];
     }
+    } while (kMode == 2);
+}
+
+// Whether the pairs sorted by their high digits alone are in order.
+__global__ void __launch_bounds__(256) k_order(const uint64_t* __restrict__ first_k, const uint64_t* __restrict__ second_k,
+                                               size_t n, SortPlan* plan, int passes) {
+    const int defer = (int)plan->defer;
+    if (defer == 0) return;
+    const uint64_t* __restrict__ k = (passes - defer) & 1 ? second_k : first_k;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    bool bad = false;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += stride) bad = bad || k[i] < k[i - 1];
+    if (__syncthreads_or(bad) && threadIdx.x == 0) plan->unsorted = 1u;
+}
+
+// The status words of the passes that have run, cleared for the passes put on after all.
+__global__ void __launch_bounds__(256) k_status_clear(const SortPlan* plan, uint4* __restrict__ status, size_t words4) {
+    if (!plan->unsorted) return;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words4; i += stride) status[i] = uint4{0, 0, 0, 0};
+}
+
+// The sorted pairs back from the second buffers where an odd number of passes has run.
+__global__ void __launch_bounds__(256) k_home(uint64_t* __restrict__ first_k, uint32_t* __restrict__ first_v,
+                                              const uint64_t* __restrict__ second_k,
+                                              const uint32_t* __restrict__ second_v, size_t n, const SortPlan* plan,
+                                              int passes) {
+    const int ran = passes - (int)plan->defer + (plan->unsorted ? passes : 0);
+    if (!(ran & 1)) return;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        first_k[i] = second_k[i];
+        first_v[i] = second_v[i];
+    }
 }
 
 // A pass of one tile is a chain of latencies (about 11,800 cycles at 12 keys per thread: 4,000 rank
@@ -289,6 +374,18 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
 // passes overlapped too; 3,000 63-bit keys 85 -> 42, 240,000 117 -> 89, 1,000,000 180 -> 176, and
 // 1,500,000, whose tiles no longer fit at once, 224 -> 225.
 constexpr size_t kSmallSort = 1u << 20;
+
+// Anchor keys of cells far above the key's depth: their low digits are set by the high ones (the
+// walk down to a cell's first corner), so that sorting by the high digits sorts them.  A large sort
+// of many passes looks: low passes that meet at most kFewDigits digits (every digit turns up in keys
+// spread over them) are left out, the result is checked, and if it is not in order every pass
+// runs, from the order reached: ties there are in input order, so the result is the same.  All of it
+// is decided on the device: the sort stays asynchronous.  63-bit keys of 30-bit cells: 15,074,927 in
+// 1,225 us before, 786 now, 4 M 379 and 290, 2.5 M 260 and 216.  Keys that fill their digits pay for
+// the launches that find nothing to do, 10 us or so (4 M: 462 before, 470 now), which the rule keeps
+// to sorts that are long beside it: 1.5 M would take 250 without and 281 with.
+constexpr size_t kPlannedSort = 2u << 20;
+constexpr int kPlannedPasses = 6;
 
 // Bytes of one pass's tile status words and ticket, for every shape: at most
 // ceil(n / smallest tile) tiles of at most kMaxRadix digits (9-bit digits on the
@@ -313,17 +410,23 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
     uint64_t* kalt = (uint64_t*)p; p += fl_align256(n * 8);
     uint32_t* valt = (uint32_t*)p; p += fl_align256(n * 4);
     uint32_t* hist = (uint32_t*)p; p += fl_align256((size_t)kMaxPasses * kMaxRadix * 4);
-    unsigned* done = (unsigned*)p; p += 256;
+    SortPlan* plan = (SortPlan*)p; p += 256;
     char* stat0 = p;
     const size_t stat_stride = fl_align256(tiles * R * 4 + 4);  // at most status_stride_min(n)
     // clear histograms, their block count and the per-pass status/tickets in one memset
     FL_TRY_CUDA(ctx, cudaMemsetAsync(hist, 0, fl_align256((size_t)kMaxPasses * kMaxRadix * 4) + 256 + passes * stat_stride,
                                      ctx->stream), "sort clear");
     constexpr size_t smem = onesweep_smem<kThreads, kBits, kItems>();
-    FL_TRY_CUDA(ctx, cudaFuncSetAttribute(k_onesweep<kThreads, kBits, kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem), "sort shared memory");
+    constexpr bool kCanPlan = kItems == kLargeItems;
+    const bool planned = kCanPlan && n >= kPlannedSort && passes >= kPlannedPasses;
+    constexpr int kPlannedMode = kCanPlan ? 1 : 0, kLateMode = kCanPlan ? 2 : 0;  // only large tiles have these modes
+    const auto kernel = planned ? k_onesweep<kThreads, kBits, kItems, kPlannedMode> : k_onesweep<kThreads, kBits, kItems, 0>;
+    const auto late = k_onesweep<kThreads, kBits, kItems, kLateMode>;
+    FL_TRY_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                "sort shared memory");
     unsigned hb = fl_blocks(n, 256, ctx->num_sms * 4);
-    k_histogram<kBits><<<hb, 256, 0, ctx->stream>>>(keys, n, begin_bit, end_bit, passes, hist, done);
+    (planned ? k_histogram<kBits, true> : k_histogram<kBits, false>)<<<hb, 256, 0, ctx->stream>>>(
+        keys, n, begin_bit, end_bit, passes, hist, plan);
     FL_CHECK_LAUNCH(ctx, "k_histogram");
     cudaLaunchAttribute early{};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -337,18 +440,37 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
     cfg.numAttrs = 1;
     uint64_t* ks[2] = {keys, kalt};
     uint32_t* vs[2] = {vals, valt};
-    int cur = 0;
-    for (int ps = 0; ps < passes; ++ps) {
+    int cur = 0;  // of a planned sort the kernels work out the buffers
+    auto launch = [&](decltype(kernel) k, int ps) -> int {
         uint32_t* status = (uint32_t*)(stat0 + ps * stat_stride);
         unsigned* ticket = (unsigned*)(status + tiles * R);
         int sh = begin_bit + kBits * ps;
-        const uint64_t* kin = ks[cur];
-        const uint32_t* vin = vs[cur];
         const uint32_t* offs = hist + ps * R;
-        cudaLaunchKernelEx(&cfg, k_onesweep<kThreads, kBits, kItems>, kin, vin, ks[cur ^ 1], vs[cur ^ 1], n, sh,
-                           digit_mask(end_bit, sh, kBits), offs, status, ticket, ctx->dev_status);
+        cudaLaunchKernelEx(&cfg, k, ks[cur], vs[cur], ks[cur ^ 1], vs[cur ^ 1], n, sh, digit_mask(end_bit, sh, kBits), offs,
+                           status, ticket, ctx->dev_status, (const SortPlan*)plan, ps, passes);
         FL_CHECK_LAUNCH(ctx, "k_onesweep");
-        cur ^= 1;
+        if (!planned) cur ^= 1;
+        return FL_OK;
+    };
+    for (int ps = 0; ps < passes; ++ps) {
+        const int rc = launch(kernel, ps);
+        if (rc) return rc;
+    }
+    if (planned) {
+        const unsigned grid = fl_blocks(n, 256, ctx->num_sms * 8);
+        k_order<<<grid, 256, 0, ctx->stream>>>(keys, kalt, n, plan, passes);
+        FL_CHECK_LAUNCH(ctx, "k_order");
+        k_status_clear<<<ctx->num_sms, 256, 0, ctx->stream>>>(plan, (uint4*)stat0, passes * stat_stride / 16);
+        FL_CHECK_LAUNCH(ctx, "k_status_clear");
+        FL_TRY_CUDA(ctx, cudaFuncSetAttribute(late, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                    "sort shared memory");
+        cfg.gridDim = dim3((unsigned)ctx->num_sms * (kThreads == 512 ? 2 : (kBits == 8 ? 4 : 3)));
+        for (int ps = 0; ps < passes; ++ps) {
+            const int rc = launch(late, ps);
+            if (rc) return rc;
+        }
+        k_home<<<grid, 256, 0, ctx->stream>>>(keys, vals, kalt, valt, n, plan, passes);
+        FL_CHECK_LAUNCH(ctx, "k_home");
     }
     if (cur == 1) {
         FL_TRY_CUDA(ctx, cudaMemcpyAsync(keys, kalt, n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "sort copy");
