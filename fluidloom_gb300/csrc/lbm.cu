@@ -2400,13 +2400,15 @@ void launch_class(fl_ctx* ctx, fl_pool* P, StepArgs a, int l, int kind, cudaStre
             if (sums) k_collide_staged<true, false, true><<<grid, 128, stage_bytes(true, false), st>>>(a, P->nb27);
             else k_collide_staged<true, false, false><<<grid, 128, stage_bytes(true, false), st>>>(a, P->nb27);
         } else {
-            // A level of a few waves of general bricks is bound by latency: programmatic launch, so
-            // that the blocks' lists, rows and gathers, which k_interface does not write, overlap its
-            // run; the values are waited for inside the kernel.  20 steps of a 32^3 cavity (one wave)
-            // 916 -> 847 us, monitored obstacles (2,900 bricks) 1,411 -> 1,365; with it for every
-            // size 24 cavities (24,000 bricks) 4,585 -> 4,640.
+            // A pool of a few waves of bricks is bound by latency: programmatic launch, so that the
+            // blocks' lists, rows and gathers, which k_interface does not write, overlap its run; the
+            // values are waited for inside the kernel.  20 steps of a 32^3 cavity (one wave) 916 -> 847
+            // us, monitored obstacles (2,900 bricks) 1,411 -> 1,365.  Beside levels that fill the GPU
+            // the early blocks only keep theirs out: 3 steps past a sphere, base edge 32, 3 levels, 1,847 us
+            // without it, 1,880 with it on its small levels; 24 cavities (24,000 bricks) 4,585 and
+            // 4,640 with it for every size.
             const uint32_t* nb27 = P->nb27;
-            if (dd1 > dd0 && cnt <= 4 * grid) {
+            if (dd1 > dd0 && P->mesh.num_cells <= 32u * (size_t)ctx->num_sms) {
                 cudaLaunchAttribute early{};
                 early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
                 early.val.programmaticStreamSerializationAllowed = 1;
