@@ -104,7 +104,7 @@ int fl_collect_device_status(fl_ctx* ctx, const char* what) {
 
 // The context's own memory pool.  CUDA's default pool hands every free block back to the system
 // whenever a stream is synchronised, so a regrid, which replaces its mesh's columns, mapped and
-// unmapped them each time (a 20 M-leaf regrid 9,180 -> 7,680 us, with the small reads through pinned
+// unmapped them each time (a 25 M-leaf regrid 9,180 -> 7,680 us, with the small reads through pinned
 // memory); this one keeps up to a 64th of the device's memory between calls and gives all of it
 // back with the context, or when an allocation would fail for want of it.
 static int create_pool(fl_ctx* c) {

@@ -346,7 +346,7 @@ __device__ __forceinline__ bool in_domain(const Octree& T, int32_t x, int32_t y,
 
 // Exclusive prefix of v over the block in thread order (256 threads), the block's total added to
 // *counter: the block's share starts at the returned base.  One atomic per block: a same-address
-// atomic per warp alone took 0.3 ms for 20 M leaves.
+// atomic per warp alone took 0.3 ms for 25 M leaves.
 __device__ __forceinline__ uint32_t block_claim(uint32_t v, uint32_t* counter) {
     __shared__ uint32_t s_sum[8], s_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -254,11 +254,6 @@ __global__ void __launch_bounds__(kThreads) k_compact_keep(const uint64_t* __res
     }
 }
 
-__global__ void k_fill_u32(uint32_t* p, uint32_t v, size_t n) {
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = v;
-}
-
 __global__ void k_invert_perm(const uint32_t* __restrict__ sorted_ids, uint32_t m, uint32_t* __restrict__ perm) {
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += stride) perm[sorted_ids[j]] = (uint32_t)j;
@@ -309,13 +304,6 @@ int fl_scan_u32_with(fl_ctx* ctx, const uint32_t* in, uint32_t* out, size_t n, u
     else
         k_scan<false><<<(unsigned)tiles, kThreads, 0, ctx->stream>>>(in, out, n, status, ticket, total, ctx->dev_status);
     FL_CHECK_LAUNCH(ctx, "k_scan");
-    return FL_OK;
-}
-
-int fl_launch_fill_u32(fl_ctx* ctx, uint32_t* p, uint32_t v, size_t n) {
-    if (!n) return FL_OK;
-    k_fill_u32<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(p, v, n);
-    FL_CHECK_LAUNCH(ctx, "k_fill_u32");
     return FL_OK;
 }
 

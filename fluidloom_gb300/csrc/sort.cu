@@ -49,7 +49,7 @@ struct SortPlan {
 };
 constexpr uint32_t kFewDigits = 32;
 
-// Every pass's histogram, then, in the block that finishes last (*done counts the
+// Every pass's histogram, then, in the block that finishes last (plan->done counts the
 // blocks, starting at 0), each pass's bins scanned in place to exclusive offsets: a
 // warp per pass, R / 32 consecutive bins a lane.  With kPlanned it also puts off
 // the low passes that meet at most kFewDigits different digits.
