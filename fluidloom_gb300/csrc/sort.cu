@@ -333,15 +333,17 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
     } while (kMode == 2);
 }
 
-// Whether the pairs sorted by their high digits alone are in order.
+// Whether the pairs sorted by their high digits alone are in order (of the sorted bits: begin_bit up,
+// as many as mask has).
 __global__ void __launch_bounds__(256) k_order(const uint64_t* __restrict__ first_k, const uint64_t* __restrict__ second_k,
-                                               size_t n, SortPlan* plan, int passes) {
+                                               size_t n, SortPlan* plan, int passes, int begin_bit, uint64_t mask) {
     const int defer = (int)plan->defer;
     if (defer == 0) return;
     const uint64_t* __restrict__ k = (passes - defer) & 1 ? second_k : first_k;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     bool bad = false;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += stride) bad = bad || k[i] < k[i - 1];
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += stride)
+        bad = bad || ((k[i] >> begin_bit) & mask) < ((k[i - 1] >> begin_bit) & mask);
     if (__syncthreads_or(bad) && threadIdx.x == 0) plan->unsorted = 1u;
 }
 
@@ -458,7 +460,8 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
     }
     if (planned) {
         const unsigned grid = fl_blocks(n, 256, ctx->num_sms * 8);
-        k_order<<<grid, 256, 0, ctx->stream>>>(keys, kalt, n, plan, passes);
+        k_order<<<grid, 256, 0, ctx->stream>>>(keys, kalt, n, plan, passes, begin_bit,
+                                               end_bit - begin_bit >= 64 ? ~0ull : (1ull << (end_bit - begin_bit)) - 1);
         FL_CHECK_LAUNCH(ctx, "k_order");
         k_status_clear<<<ctx->num_sms, 256, 0, ctx->stream>>>(plan, (uint4*)stat0, passes * stat_stride / 16);
         FL_CHECK_LAUNCH(ctx, "k_status_clear");

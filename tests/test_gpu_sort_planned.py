@@ -44,3 +44,29 @@ def test_sort_puts_passes_off(ctx, n, bits, what, shape):
         np.testing.assert_array_equal(dk.to_host(), keys[order])
     finally:
         ctx.call("fl_sort_set_config", 8, 256)
+
+
+@pytest.mark.parametrize("swap", [False, True])
+@pytest.mark.parametrize("bits", [(0, 56), (5, 61), (8, 64)])
+def test_bits_beside_the_sorted_ones(ctx, bits, swap):
+    """Bits outside the range take no part: in the order that is checked either.  One pair differs only in
+    the range's lowest bit, against the bits above the range (or below it)."""
+    n, (lo, hi) = PLANNED + 5, bits
+    rng = np.random.default_rng(lo)
+    top = rng.permutation(n).astype(np.uint64) << np.uint64(1)
+    part = top << np.uint64(hi - lo - 23)  # unique but for the pair; every low bit 0
+    a, b = n // 3, 2 * n // 3
+    part[b] = part[a]
+    part[b if swap else a] |= np.uint64(1)
+    keys = part << np.uint64(lo)
+    if hi < 64:  # the keys as a whole are in order once the high digits are
+        above = part > (part[a] | np.uint64(1))
+        above[b] = True
+        keys[above] |= np.uint64(1) << np.uint64(hi)
+    if lo:
+        keys |= rng.integers(0, 1 << lo, n, dtype=np.uint64)
+    order = np.argsort(part, kind="stable")
+    dk, di = DeviceArray.from_host(ctx, keys), DeviceArray.from_host(ctx, np.arange(n, dtype=np.uint32))
+    ctx.call("fl_sort_pairs_u64_u32", dk.ptr, di.ptr, ctypes.c_size_t(n), *bits)
+    np.testing.assert_array_equal(di.to_host(), order.astype(np.uint32))
+    np.testing.assert_array_equal(dk.to_host(), keys[order])
