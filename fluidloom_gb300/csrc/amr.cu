@@ -299,7 +299,10 @@ __device__ __forceinline__ bool merge_candidate(const fl_mesh_dev& m, size_t i, 
 
 // Lane c < 8 of a warp: sibling c of candidate i (the leaf holding its anchor
 // point, if that leaf has the octet's level), FL_INVALID_INDEX otherwise;
-// `ok` tells whether it is a mergeable member (flag -1, FLUID).
+// `ok` tells whether it is a mergeable member (flag -1, FLUID).  Of a leaf that
+// a mesh lists more than once the search finds one copy, so sibling 0 is a
+// member only as the candidate itself: an octet has one leader however often its
+// first sibling is listed, no leaf is in two groups, and there are at most n / 8.
 __device__ __forceinline__ uint32_t sibling_of(const fl_probe& P, const fl_mesh_dev& m, const fl_domain_dev& dom,
                                                size_t i, int c, bool* ok) {
     const int l = m.level[i];
@@ -309,7 +312,7 @@ __device__ __forceinline__ uint32_t sibling_of(const fl_probe& P, const fl_mesh_
                    sz = (uint32_t)(m.z[i] | ((c >> 2) & 1)) << sh;
     uint32_t j = fl_probe_point(P, m.case_id != nullptr, cs, sx, sy, sz);
     if (j != FL_INVALID_INDEX && m.level[j] != l) j = FL_INVALID_INDEX;
-    *ok = j != FL_INVALID_INDEX && m.flags[j] == -1 && m.state[j] == 0;
+    *ok = j != FL_INVALID_INDEX && (c > 0 || j == (uint32_t)i) && m.flags[j] == -1 && m.state[j] == 0;
     return j;
 }
 
@@ -319,17 +322,20 @@ __device__ __forceinline__ uint32_t sibling_of(const fl_probe& P, const fl_mesh_
 // before the candidate, h = the candidate's Hilbert digit at its level (read
 // from its run key).  Lane c takes the c-th of them, in key order; it is a
 // member when it is a leaf of the candidate's level under the same parent
-// (case, x >> 1, y >> 1, z >> 1).  Eight members <=> the eight children are
-// leaves of that level <=> sibling_of finds all eight; `ok` as there.  The
-// members come in key order, not by child position (their child bits say
-// which is which).
+// (case, x >> 1, y >> 1, z >> 1) with the Hilbert digit c, so that eight members
+// are the eight children (a mesh with repeated leaves has run order ids, but
+// a caller that vouches for the key order is not checked).  Eight members <=> the
+// eight children are leaves of that level <=> sibling_of finds all eight; `ok`
+// as there.  The members come in key order, not by child position (their child
+// bits say which is which).
 __device__ __forceinline__ uint32_t sibling_in_run(const fl_probe& P, const fl_mesh_dev& m, size_t i, int c, bool* ok) {
     const int l = m.level[i];
-    const int h = (int)((__ldg((const unsigned long long*)(P.L.keys + i)) >> (3 * (P.top - l))) & 7u);
+    auto digit = [&](size_t j) { return (int)((__ldg((const unsigned long long*)(P.L.keys + j)) >> (3 * (P.top - l))) & 7u); };
+    const int h = digit(i);
     *ok = false;
     if (i < (size_t)h) return FL_INVALID_INDEX;
     const size_t j = i - h + c;
-    if (j >= m.n || m.level[j] != l || (m.x[j] >> 1) != (m.x[i] >> 1) || (m.y[j] >> 1) != (m.y[i] >> 1) ||
+    if (j >= m.n || m.level[j] != l || digit(j) != c || (m.x[j] >> 1) != (m.x[i] >> 1) || (m.y[j] >> 1) != (m.y[i] >> 1) ||
         (m.z[j] >> 1) != (m.z[i] >> 1) || (m.case_id && m.case_id[j] != m.case_id[i]))
         return FL_INVALID_INDEX;
     *ok = m.flags[j] == -1 && m.state[j] == 0;
@@ -358,7 +364,7 @@ __device__ __forceinline__ uint32_t sibling_in_run(const fl_probe& P, const fl_m
 // found (*groups counts them; group_of holds FL_INVALID_INDEX before), which a
 // regrid, where only the emission reads the numbers, need not fix: 25 M cells
 // a scan and a second pass less (a regrid and neighbour rows 3,005 us, 2,897 now).
-// In group_of, a leader's group (there are at most n / 8 < 2^29) -- so the entries with the top bit, the
+// In group_of, a leader's group (there are at most n / 8 < 2^29: sibling_of) -- so the entries with the top bit, the
 // leaders' and FL_INVALID_INDEX of the cells in no group, are those of the cells that make a new one.
 constexpr uint32_t kLeads = 0x80000000u;
 
@@ -487,7 +493,7 @@ __global__ void __launch_bounds__(kT) k_leaders(fl_mesh_dev m, fl_domain_dev dom
 // at a time (lane 8s + c: sibling c of the s-th).
 __global__ void __launch_bounds__(kT) k_members(fl_mesh_dev m, fl_domain_dev dom, fl_locator L,
                                                 const uint32_t* __restrict__ is_leader,
-                                                   const uint32_t* __restrict__ gid, uint32_t* __restrict__ members,
+                                                const uint32_t* __restrict__ gid, uint32_t* __restrict__ members,
                                                 uint32_t* __restrict__ group_of) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];

@@ -171,13 +171,13 @@ __global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__
 // encoded at depth - cut levels, the low 3(A - l - cut) bits cleared (the case
 // id above bit 3 * (depth - cut)).
 //
-// unsorted (when given) is set when some run start is smaller than the one
-// before it.  A warp takes a range of consecutive leaves and keeps the last of
+// order (when given) gets bit 0 when some run start is smaller than the one
+// before it, bit 1 when some is the same (a leaf listed twice, or overlapping leaves).  A warp takes a range of consecutive leaves and keeps the last of
 // 32 for the next 32, so only the start of its range is encoded twice (25 M
 // leaves: 107 us and a pass of 41 over the keys, 135 now).
 __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev dom, int cut,
                                                   const uint32_t* __restrict__ deepest, uint64_t* __restrict__ keys,
-                                                  uint32_t* __restrict__ unsorted) {
+                                                  uint32_t* __restrict__ order) {
     __shared__ __align__(16) uint8_t t1[96];
     __shared__ __align__(16) uint16_t t3c[12 * 512];
     fl_keys_fill_tables_cat(t1, t3c);
@@ -198,20 +198,22 @@ __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev d
     const size_t first = ((size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per;
     if (first >= m.n) return;
     const size_t end = min(first + per, m.n);
-    uint64_t last = unsorted && first ? key_of(first - 1) : 0;
-    bool bad = false;
+    uint64_t last = order && first ? key_of(first - 1) : 0;
+    unsigned bad = 0u;
     for (size_t i0 = first; i0 < end; i0 += 32) {
         const size_t i = i0 + lane;
         const uint64_t k = i < end ? key_of(i) : ~0ull;
         if (i < end) keys[i] = k;
-        if (unsorted) {
+        if (order) {
             uint64_t before = __shfl_up_sync(0xFFFFFFFFu, k, 1);
             if (lane == 0) before = last;
-            bad = bad || k < before;
+            bad |= k < before ? 1u : 0u;
+            bad |= k == before && i > 0 && i < end ? 2u : 0u;
             last = __shfl_sync(0xFFFFFFFFu, k, 31);
         }
     }
-    if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) *unsorted = 1u;
+    bad = __reduce_or_sync(0xFFFFFFFFu, bad);
+    if (bad && lane == 0) atomicOr(order, bad);
 }
 
 __global__ void k_iota(uint32_t* __restrict__ ids, size_t n) {
@@ -647,7 +649,7 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
     *L = fl_locator{keys, nullptr, dir, m.level, n, log2nb, 0};
     if (n == 0) return FL_OK;
     FL_TRY_CUDA(ctx, cudaMemsetAsync(flag, 0, 12, ctx->stream), "locator");
-    uint32_t hf[2] = {0, (uint32_t)std::max(level_bound, 0)};  // unsorted, deepest level
+    uint32_t hf[2] = {0, (uint32_t)std::max(level_bound, 0)};  // order (k_run_keys), deepest level
     if (level_bound < 0) {
         k_level_range<<<fl_blocks((n + 15) / 16, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m.level, n, flag + 1);
         FL_CHECK_LAUNCH(ctx, "k_level_range");
@@ -661,13 +663,17 @@ int fl_locator_build(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom
         if (rc) return rc;
     }
     L->cut = std::max(dom.anchor_level - (int)hf[1], 0);
-    if (hf[0]) {  // stable: equal run starts keep mesh order, so the last of them is found
+    // Stable: equal run starts keep mesh order, so the last of them is found.  A mesh in key order that
+    // has some gets ids too, its own order: octets are not consecutive there, and want the search.
+    if (hf[0]) {
         k_iota<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(ids, n);
         FL_CHECK_LAUNCH(ctx, "k_iota");
-        // the keys hold 3 (depth - cut) bits, plus 16 for case ids
-        const int end_bit = std::min(64, 3 * (dom.depth - L->cut) + (m.case_id ? 16 : 0));
-        int rc = fl_sort_pairs_with(ctx, keys, ids, n, 0, end_bit, p);
-        if (rc) return rc;
+        if (hf[0] & 1u) {
+            // the keys hold 3 (depth - cut) bits, plus 16 for case ids
+            const int end_bit = std::min(64, 3 * (dom.depth - L->cut) + (m.case_id ? 16 : 0));
+            int rc = fl_sort_pairs_with(ctx, keys, ids, n, 0, end_bit, p);
+            if (rc) return rc;
+        }
         L->ids = ids;
     }
     if (!probed && !L->ids) return FL_OK;  // octets in key order are found without a search
