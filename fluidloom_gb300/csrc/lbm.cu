@@ -1768,6 +1768,9 @@ struct fl_pool {
     cudaGraphExec_t graph_solid[2] = {nullptr, nullptr};
     uint64_t graph_solid_kernels[2] = {0, 0};
     bool graph_solid_ok[2] = {false, false};
+    // the launches of the step emitted last, in order (a word each: level, class and variant), and
+    // those that each graph was captured from
+    std::vector<uint32_t> launched, graph_shape[2], graph_solid_shape[2];
     uint64_t version = 0;                           // bumped whenever the emitted launches change
     void* adapt_scratch = nullptr;
     size_t adapt_scratch_bytes = 0;
@@ -1923,7 +1926,7 @@ int alloc_brick_arrays_beside(fl_ctx* ctx, fl_pool* P, size_t cap, BrickArrays* 
 }
 
 // The captured steps no longer match the pool: mark them stale.  The next
-// capture updates the instantiated graph in place when its shape is unchanged
+// capture updates the instantiated graph in place when it holds the same launches
 // (cudaGraphExecUpdate) instead of instantiating anew.  Every change of the
 // bricks or populations passes here, so it also makes each level write its
 // all-solid bricks for its next two sub-steps (both buffers).
@@ -2377,7 +2380,11 @@ void launch_class(fl_ctx* ctx, fl_pool* P, StepArgs a, int l, int kind, cudaStre
     }
     a.list = P->list + off;
     a.count = cnt;
-    ctx->launches += (kind == 1 && P->lvl_desc[l + 1] > P->lvl_desc[l]) ? 2 : 1;
+    const bool described = kind == 1 && P->lvl_desc[l + 1] > P->lvl_desc[l];
+    const bool early = described && !P->staging && P->mesh.num_cells <= 32u * (size_t)ctx->num_sms;
+    P->launched.push_back((uint32_t)l | (uint32_t)kind << 8 | (uint32_t)P->staging << 10 | (merged ? 1u << 12 : 0u) |
+                          (described ? 1u << 13 : 0u) | (early ? 1u << 14 : 0u) | (a.part ? 1u << 15 : 0u));
+    ctx->launches += described ? 2 : 1;
     const bool sums = a.part != nullptr;
     if (kind == 0) {
         unsigned grid = std::min<unsigned>(cnt, (unsigned)ctx->num_sms * P->grid_mult);
@@ -2391,7 +2398,7 @@ void launch_class(fl_ctx* ctx, fl_pool* P, StepArgs a, int l, int kind, cudaStre
     } else if (kind == 1) {
         a.desc_off = P->slow_off + P->cls_off[1][l];
         const uint32_t dd0 = P->lvl_desc[l], dd1 = P->lvl_desc[l + 1];
-        if (dd1 > dd0) k_interface<<<fl_blocks(dd1 - dd0, 256, ctx->num_sms * 8), 256, 0, st>>>(a, dd0, dd1, P->pv);
+        if (described) k_interface<<<fl_blocks(dd1 - dd0, 256, ctx->num_sms * 8), 256, 0, st>>>(a, dd0, dd1, P->pv);
         const unsigned grid = std::min<unsigned>(cnt, (unsigned)ctx->num_sms * 4);
         if (P->staging == 2) {
             if (sums) k_collide_staged<true, true, true><<<grid, 128, stage_bytes(true, true), st>>>(a, P->nb27);
@@ -2408,7 +2415,7 @@ void launch_class(fl_ctx* ctx, fl_pool* P, StepArgs a, int l, int kind, cudaStre
             // without it, 1,880 with it on its small levels; 24 cavities (24,000 bricks) 4,585 and
             // 4,640 with it for every size.
             const uint32_t* nb27 = P->nb27;
-            if (dd1 > dd0 && P->mesh.num_cells <= 32u * (size_t)ctx->num_sms) {
+            if (early) {
                 cudaLaunchAttribute early{};
                 early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
                 early.val.programmaticStreamSerializationAllowed = 1;
@@ -2500,6 +2507,7 @@ void step_level(fl_ctx* ctx, fl_pool* P, int l, int sub, LaunchTimer* tm, Dag* d
 // One level-0 step: in order on the context stream, or as the dependency graph
 // forked from and joined back into the context stream.
 void level0_step(fl_ctx* ctx, fl_pool* P, LaunchTimer* tm = nullptr) {
+    P->launched.clear();
     if (tm || P->streams < 2) {
         step_level(ctx, P, 0, 0, tm, nullptr, true);
         return;
@@ -2724,6 +2732,7 @@ int fl_pool_step(fl_ctx* ctx, fl_pool* P, int nsteps) {
         cudaGraphExec_t* exec = settled ? &P->graph[p0] : &P->graph_solid[p0];
         bool* ok = settled ? &P->graph_ok[p0] : &P->graph_solid_ok[p0];
         uint64_t* kernels = settled ? &P->graph_kernels[p0] : &P->graph_solid_kernels[p0];
+        std::vector<uint32_t>& shape = settled ? P->graph_shape[p0] : P->graph_solid_shape[p0];
         if (!*ok) {
             int saved[16];
             std::memcpy(saved, P->parity, sizeof(saved));
@@ -2741,10 +2750,13 @@ int fl_pool_step(fl_ctx* ctx, fl_pool* P, int nsteps) {
             std::memcpy(P->parity, saved, sizeof(saved));
             std::memcpy(P->solid_due, saved_due, sizeof(saved_due));
             FL_TRY_CUDA(ctx, e, "capture end");
+            // An update keeps the executable's edges: with other launches than it was captured from, a kernel
+            // that does not wait for the one before it could end up behind a programmatic edge, where
+            // that one starts it early (k_interface).  So only the same launches are updated.
             bool updated = false;
             if (*exec) {
                 cudaGraphExecUpdateResultInfo info;
-                updated = cudaGraphExecUpdate(*exec, g, &info) == cudaSuccess;
+                updated = shape == P->launched && cudaGraphExecUpdate(*exec, g, &info) == cudaSuccess;
                 if (!updated) {
                     cudaGetLastError();  // a failed update leaves no sticky error; clear the last one
                     cudaGraphExecDestroy(*exec);
@@ -2752,6 +2764,7 @@ int fl_pool_step(fl_ctx* ctx, fl_pool* P, int nsteps) {
                 }
             }
             if (!updated) e = cudaGraphInstantiate(exec, g, 0);
+            shape = P->launched;
             cudaGraphDestroy(g);
             FL_TRY_CUDA(ctx, e, "graph instantiate");
             *ok = true;
