@@ -626,27 +626,31 @@ __global__ void __launch_bounds__(128, 4) k_collide_general(StepArgs a, const ui
         gather_quad<0, Q>(a, s_nb, x0, y, z, f);
         if (kEarly) cudaGridDependencySynchronize();  // k_interface's values are there (returns at once later on)
         const float* pv = a.pv + (tables ? a.desc_off[w - a.plain] : 0u);
+        // Launched early, the values are still written while the kernel runs: ordinary loads, to which the
+        // wait above makes them visible.  The read-only path (__ldg) is for data that nobody writes in a
+        // kernel's lifetime; it could hold a line from before, of another level's values beside these.
+        // (__ldcg, volatile and past L1, took 2.7 % of a 32^3 cavity's step.)
         uint32_t r = qm.w;
         if (qm.x) {
 #pragma unroll
             for (int q = 0; q < 8; ++q)
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    if ((qm.x >> (q * 4 + i)) & 1u) f[q][i] = __ldg(pv + r++);
+                    if ((qm.x >> (q * 4 + i)) & 1u) f[q][i] = kEarly ? pv[r++] : __ldg(pv + r++);
         }
         if (qm.y) {
 #pragma unroll
             for (int q = 8; q < 16; ++q)
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    if ((qm.y >> (q * 4 + i - 32)) & 1u) f[q][i] = __ldg(pv + r++);
+                    if ((qm.y >> (q * 4 + i - 32)) & 1u) f[q][i] = kEarly ? pv[r++] : __ldg(pv + r++);
         }
         if (qm.z) {
 #pragma unroll
             for (int q = 16; q < Q; ++q)
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    if ((qm.z >> (q * 4 + i - 64)) & 1u) f[q][i] = __ldg(pv + r++);
+                    if ((qm.z >> (q * 4 + i - 64)) & 1u) f[q][i] = kEarly ? pv[r++] : __ldg(pv + r++);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
