@@ -137,9 +137,8 @@ __host__ __device__ constexpr size_t onesweep_smem() {
 // fit the GPU, a tile after another: most sorts need none of these, and so small a grid ends soonest.
 template <int kThreads, int kBits, int kItems, int kMode>
 __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 4 : 3))
-    k_onesweep(uint64_t* __restrict__ first_k, uint32_t* __restrict__ first_v, uint64_t* __restrict__ second_k,
-               uint32_t* __restrict__ second_v, size_t n, int shift, uint32_t dmask,
-               const uint32_t* __restrict__ bin_off, uint32_t* status, unsigned* ticket, uint32_t* dev_status,
+    k_onesweep(uint64_t* first_k, uint32_t* first_v, uint64_t* second_k, uint32_t* second_v, size_t n, int shift, uint32_t dmask,
+               const uint32_t* bin_off, uint32_t* status, unsigned* ticket, uint32_t* dev_status,
                const SortPlan* plan, int pass, int passes) {
     constexpr int R = 1 << kBits;
     constexpr int kWarps = kThreads / 32;
@@ -172,10 +171,14 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
         if (kMode == 1 ? pass < defer : !ld_vol(&plan->unsorted)) return;
         swapped = kMode == 1 ? (pass - defer) & 1 : (passes - defer + pass) & 1;
     }
-    const uint64_t* __restrict__ kin = swapped ? second_k : first_k;
-    const uint32_t* __restrict__ vin = swapped ? second_v : first_v;
-    uint64_t* __restrict__ kout = swapped ? first_k : second_k;
-    uint32_t* __restrict__ vout = swapped ? first_v : second_v;
+    // The pass before wrote the input while this kernel was already resident: ordinary loads, to which the
+    // wait above makes it visible.  With __restrict__ a compiler may read buffers that a pass only reads
+    // through the read-only cache, which is for data that nobody writes in the kernel's lifetime.  (__ldcg
+    // for all of a tile before its ranking: 15,074,927 mesh keys and their sort 869 -> 940 us.)
+    const uint64_t* kin = swapped ? second_k : first_k;
+    const uint32_t* vin = swapped ? second_v : first_v;
+    uint64_t* kout = swapped ? first_k : second_k;
+    uint32_t* vout = swapped ? first_v : second_v;
     do {
     if (kMode != 0) {
         __syncthreads();
