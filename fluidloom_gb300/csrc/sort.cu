@@ -23,6 +23,8 @@
 #include "common.cuh"
 #include "scan.cuh"
 
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 namespace {
@@ -43,25 +45,34 @@ __host__ __device__ constexpr uint32_t digit_mask(int end_bit, int sh, int bits)
 }
 
 // A sort that may leave out passes keeps its state behind the histograms: the
-// histogram's block count, the low passes put off, whether they are needed.
+// histogram's block count, the low passes left out, the runs to sort by their low digits.
 struct SortPlan {
-    unsigned done, defer, unsorted;
+    unsigned done, defer, runs;
 };
 constexpr uint32_t kFewDigits = 32;
+constexpr uint32_t kShortRun = 1024;       // keys of one high part that a warp sorts by counting
+
+__host__ __device__ constexpr uint64_t range_mask(int begin_bit, int end_bit) {
+    return end_bit - begin_bit >= 64 ? ~0ull : (1ull << (end_bit - begin_bit)) - 1;
+}
 
 // Every pass's histogram, then, in the block that finishes last (plan->done counts the
 // blocks, starting at 0), each pass's bins scanned in place to exclusive offsets: a
-// warp per pass, R / 32 consecutive bins a lane.  With kPlanned it also puts off
-// the low passes that meet at most kFewDigits different digits.
+// warp per pass, R / 32 consecutive bins a lane.  With kPlanned it also leaves
+// out the low passes that meet at most kFewDigits different digits, and clears the
+// table of k_sample.
 template <int kBits, bool kPlanned>
 __global__ void __launch_bounds__(256) k_histogram(const uint64_t* __restrict__ keys, size_t n, int begin_bit,
-                                                   int end_bit, int passes, uint32_t* hist, SortPlan* plan) {
+                                                   int end_bit, int passes, uint32_t* hist, SortPlan* plan,
+                                                   uint64_t* table, size_t slots) {
     constexpr int R = 1 << kBits;
     __shared__ uint32_t h[kMaxPasses][R];
     __shared__ bool last;
     for (int i = threadIdx.x; i < kMaxPasses * R; i += blockDim.x) (&h[0][0])[i] = 0;
     __syncthreads();
     size_t stride = (size_t)gridDim.x * blockDim.x;
+    if (kPlanned)
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += stride) table[i] = ~0ull;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         uint64_t k = keys[i];
         for (int p = 0; p < passes; ++p) {
@@ -122,6 +133,25 @@ __global__ void __launch_bounds__(256) k_histogram(const uint64_t* __restrict__ 
 
 __device__ __forceinline__ uint32_t ld_vol(const uint32_t* p) { return *(volatile const uint32_t*)p; }
 
+// Before the passes: keys at random places meet in a table by what is above the digits left
+// out.  Two with one high part and different low ones put the digit of their highest
+// different bit, and those above, back among the passes.
+template <int kBits>
+__global__ void __launch_bounds__(256) k_sample(const uint64_t* __restrict__ keys, size_t n, int begin_bit, uint64_t mask,
+                                                size_t samples, unsigned long long* table, int lg, SortPlan* plan) {
+    const int defer = (int)ld_vol(&plan->defer);
+    const size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (defer == 0 || w >= samples) return;
+    uint64_t h = (w + 1) * 0x9e3779b97f4a7c15ull;
+    h = (h ^ (h >> 32)) * 0x9e3779b97f4a7c15ull;
+    h = (h ^ (h >> 29)) * 0x9e3779b97f4a7c15ull;
+    const uint64_t k = (keys[__umul64hi(h, n)] >> begin_bit) & mask;
+    const uint64_t high = k >> (kBits * defer);
+    const uint64_t met = atomicExch(table + ((high * 0x9e3779b97f4a7c15ull) >> (64 - lg)), (unsigned long long)k);
+    if (met != ~0ull && met != k && met >> (kBits * defer) == high)
+        atomicMin(&plan->defer, (unsigned)((63 - __clzll((long long)(met ^ k))) / kBits));
+}
+
 // Dynamic shared memory of one onesweep tile: keys and values staged in rank
 // order, per-warp digit counters, per-digit tile offsets and global bases,
 // per-warp sums of the digit scan.
@@ -131,15 +161,13 @@ __host__ __device__ constexpr size_t onesweep_smem() {
            ((size_t)(kThreads / 32) * (1 << kBits) + 2 * (1 << kBits) + kThreads / 32) * 4;
 }
 
-// kMode 0: one pass from the first buffers into the second.  1: pass number `pass` of a sort that
-// may put passes off: nothing if this is one of them, else from the buffers where the passes run
-// before it left the pairs.  2: a pass put on after all (when the plan says so), by the blocks that
-// fit the GPU, a tile after another: most sorts need none of these, and so small a grid ends soonest.
-template <int kThreads, int kBits, int kItems, int kMode>
+// kPlanned: pass number `pass` of a sort that may leave passes out: nothing if this is one of them, else
+// from the buffers where the passes run before it left the pairs.  Otherwise from the first into the second.
+template <int kThreads, int kBits, int kItems, bool kPlanned>
 __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 4 : 3))
     k_onesweep(uint64_t* first_k, uint32_t* first_v, uint64_t* second_k, uint32_t* second_v, size_t n, int shift, uint32_t dmask,
                const uint32_t* bin_off, uint32_t* status, unsigned* ticket, uint32_t* dev_status,
-               const SortPlan* plan, int pass, int passes) {
+               const SortPlan* plan, int pass) {
     constexpr int R = 1 << kBits;
     constexpr int kWarps = kThreads / 32;
     constexpr int kTile = kThreads * kItems;
@@ -156,7 +184,9 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
     __shared__ int s_tile;
     __shared__ int s_bad;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (kMode == 0) {
+    // a tile before the wait helps the small sorts; in large ones (kPlanned: after it) 15,074,927 mesh keys
+    // took 850 us with it before, 774 after
+    if (!kPlanned) {
         if (threadIdx.x == 0) { s_tile = (int)atomicAdd(ticket, 1u); s_bad = 0; }
         for (int i = threadIdx.x; i < kWarps * R; i += kThreads) s_warp_hist[i] = 0;
     }
@@ -165,11 +195,11 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
     bool swapped = false;
-    if (kMode != 0) {
+    if (kPlanned) {
         // (every block waits above first: the pass after this one counts on the passes before)
         const int defer = (int)ld_vol(&plan->defer);
-        if (kMode == 1 ? pass < defer : !ld_vol(&plan->unsorted)) return;
-        swapped = kMode == 1 ? (pass - defer) & 1 : (passes - defer + pass) & 1;
+        if (pass < defer) return;
+        swapped = (pass - defer) & 1;
     }
     // The pass before wrote the input while this kernel was already resident: ordinary loads, to which the
     // wait above makes it visible.  With __restrict__ a compiler may read buffers that a pass only reads
@@ -179,15 +209,12 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
     const uint32_t* vin = swapped ? second_v : first_v;
     uint64_t* kout = swapped ? first_k : second_k;
     uint32_t* vout = swapped ? first_v : second_v;
-    do {
-    if (kMode != 0) {
-        __syncthreads();
+    if (kPlanned) {
         if (threadIdx.x == 0) { s_tile = (int)atomicAdd(ticket, 1u); s_bad = 0; }
         for (int i = threadIdx.x; i < kWarps * R; i += kThreads) s_warp_hist[i] = 0;
     }
     __syncthreads();
     const int tile = s_tile;
-    if (kMode == 2 && (size_t)tile * kTile >= n) return;
     const size_t tbase = (size_t)tile * kTile;
     const size_t wbase = tbase + (size_t)warp * 32 * kItems;
     const unsigned lt = (1u << lane) - 1u;
@@ -333,28 +360,124 @@ __global__ void __launch_bounds__(kThreads, kThreads == 512 ? 2 : (kBits == 8 ? 
         kout[pos] = kk;
         vout[pos] = s_vals[i];
     }
-    } while (kMode == 2);
 }
 
-// Whether the pairs sorted by their high digits alone are in order (of the sorted bits: begin_bit up,
-// as many as mask has).
+// The pairs sorted by their high digits alone, where they are not in order (of the sorted bits: begin_bit up,
+// as many as mask has): what is out of order shares its high part, so the first key of each run of one
+// high part that is not in order goes into list (at most n / 2 of them).
+template <int kBits>
 __global__ void __launch_bounds__(256) k_order(const uint64_t* __restrict__ first_k, const uint64_t* __restrict__ second_k,
-                                               size_t n, SortPlan* plan, int passes, int begin_bit, uint64_t mask) {
-    const int defer = (int)plan->defer;
+                                               size_t n, SortPlan* plan, int passes, int begin_bit, uint64_t mask,
+                                               uint32_t* __restrict__ list) {
+    const int defer = (int)plan->defer, low = kBits * defer;
     if (defer == 0) return;
-    const uint64_t* __restrict__ k = (passes - defer) & 1 ? second_k : first_k;
+    const uint64_t* __restrict__ keys = (passes - defer) & 1 ? second_k : first_k;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    bool bad = false;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += stride)
-        bad = bad || ((k[i] >> begin_bit) & mask) < ((k[i - 1] >> begin_bit) & mask);
-    if (__syncthreads_or(bad) && threadIdx.x == 0) plan->unsorted = 1u;
+    auto key = [&](size_t i) { return (keys[i] >> begin_bit) & mask; };
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += stride) {
+        uint64_t k = key(i - 1);
+        if (key(i) >= k) continue;
+        // back to the run's start, or to an earlier key out of order, whose thread lists the run
+        size_t j = i - 1;
+        bool first = true;
+        while (first && j > 0) {
+            const uint64_t before = key(j - 1);
+            if (before >> low != k >> low) break;
+            first = before <= k;
+            k = before;
+            --j;
+        }
+        if (first) list[atomicAdd(&plan->runs, 1u)] = (uint32_t)j;
+    }
 }
 
-// The status words of the passes that have run, cleared for the passes put on after all.
-__global__ void __launch_bounds__(256) k_status_clear(const SortPlan* plan, uint4* __restrict__ status, size_t words4) {
-    if (!plan->unsorted) return;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words4; i += stride) status[i] = uint4{0, 0, 0, 0};
+// The listed runs in order, a warp each, through the buffers that the last pass read.  In a short run a
+// key's place is the number of the run's keys before it (equal ones in the order they have); a longer one
+// takes stable passes over its low bits, eight at a time.
+template <int kBits>
+__global__ void __launch_bounds__(256) k_runs(uint64_t* first_k, uint32_t* first_v, uint64_t* second_k, uint32_t* second_v,
+                                              size_t n, const SortPlan* plan, int passes, int begin_bit, uint64_t mask,
+                                              const uint32_t* list) {
+    __shared__ uint32_t s_count[8][256];
+    const uint32_t runs = plan->runs;
+    const int low = kBits * (int)plan->defer, lane = threadIdx.x & 31;
+    const bool swapped = (passes - (int)plan->defer) & 1;
+    uint64_t* const keys = swapped ? second_k : first_k;
+    uint32_t* const vals = swapped ? second_v : first_v;
+    uint64_t* const tk = swapped ? first_k : second_k;
+    uint32_t* const tv = swapped ? first_v : second_v;
+    auto bits = [&](uint64_t k) { return (k >> begin_bit) & mask; };
+    uint32_t* c = s_count[threadIdx.x >> 5];
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < runs; r += warps) {
+        const size_t start = list[r];
+        const uint64_t high = bits(keys[start]) >> low;
+        uint32_t len = 0;
+        for (unsigned in = 0xFFFFFFFFu; in == 0xFFFFFFFFu;) {
+            const size_t i = start + len + lane;
+            in = __ballot_sync(0xFFFFFFFFu, i < n && bits(keys[i]) >> low == high);
+            len += in == 0xFFFFFFFFu ? 32u : (uint32_t)__ffs(~in) - 1u;
+        }
+        bool moved = true;  // the run's order is in tk, tv
+        if (len <= kShortRun) {
+            for (uint32_t e = lane; e < len; e += 32u) {
+                const uint64_t mine = bits(keys[start + e]);
+                uint32_t at = 0;
+                for (uint32_t j = 0; j < len; ++j) {
+                    const uint64_t other = bits(keys[start + j]);
+                    at += other < mine || (other == mine && j < e) ? 1u : 0u;
+                }
+                tk[start + at] = keys[start + e];
+                tv[start + at] = vals[start + e];
+            }
+        } else {
+            moved = false;
+            for (int sh = 0; sh < low; sh += 8, moved = !moved) {
+                const uint64_t* ak = (moved ? tk : keys) + start;
+                const uint32_t* av = (moved ? tv : vals) + start;
+                uint64_t* bk = (moved ? keys : tk) + start;
+                uint32_t* bv = (moved ? vals : tv) + start;
+                for (int i = lane; i < 256; i += 32) c[i] = 0u;
+                __syncwarp();
+                for (uint32_t e = lane; e < len; e += 32u) atomicAdd(&c[(bits(ak[e]) >> sh) & 255u], 1u);
+                __syncwarp();
+                uint32_t v[8], sum = 0;
+                for (int j = 0; j < 8; ++j) sum += v[j] = c[lane * 8 + j];
+                uint32_t run = sum;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, run, o);
+                    if (lane >= o) run += t;
+                }
+                run -= sum;
+                for (int j = 0; j < 8; ++j) {
+                    c[lane * 8 + j] = run;
+                    run += v[j];
+                }
+                __syncwarp();
+                for (uint32_t e0 = 0; e0 < len; e0 += 32u) {
+                    const bool in = e0 + lane < len;
+                    const uint64_t k = in ? ak[e0 + lane] : 0ull;
+                    const uint32_t d = in ? (uint32_t)(bits(k) >> sh) & 255u : 256u;
+                    const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
+                    const uint32_t base = in ? c[d] : 0u;
+                    __syncwarp();
+                    if (in && lane == __ffs(peers) - 1) c[d] = base + (uint32_t)__popc(peers);
+                    __syncwarp();
+                    if (in) {
+                        const uint32_t at = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+                        bk[at] = k;
+                        bv[at] = av[e0 + lane];
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+        for (uint32_t e = lane; moved && e < len; e += 32u) {
+            keys[start + e] = tk[start + e];
+            vals[start + e] = tv[start + e];
+        }
+    }
 }
 
 // The sorted pairs back from the second buffers where an odd number of passes has run.
@@ -362,8 +485,7 @@ __global__ void __launch_bounds__(256) k_home(uint64_t* __restrict__ first_k, ui
                                               const uint64_t* __restrict__ second_k,
                                               const uint32_t* __restrict__ second_v, size_t n, const SortPlan* plan,
                                               int passes) {
-    const int ran = passes - (int)plan->defer + (plan->unsorted ? passes : 0);
-    if (!(ran & 1)) return;
+    if (!((passes - (int)plan->defer) & 1)) return;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         first_k[i] = second_k[i];
@@ -383,12 +505,17 @@ constexpr size_t kSmallSort = 1u << 20;
 // Anchor keys of cells far above the key's depth: their low digits are set by the high ones (the
 // walk down to a cell's first corner), so that sorting by the high digits sorts them.  A large sort
 // of many passes looks: low passes that meet at most kFewDigits digits (every digit turns up in keys
-// spread over them) are left out, the result is checked, and if it is not in order every pass
-// runs, from the order reached: ties there are in input order, so the result is the same.  All of it
-// is decided on the device: the sort stays asynchronous.  63-bit keys of 30-bit cells: 15,074,927 in
-// 1,225 us before, 786 now, 4 M 379 and 290, 2.5 M 260 and 216.  Keys that fill their digits pay for
-// the launches that find nothing to do, 10 us or so (4 M: 462 before, 470 now), which the rule keeps
-// to sorts that are long beside it: 1.5 M would take 250 without and 281 with.
+// spread over them) are left out, unless a sample shows that the high digits don't decide them
+// (k_sample), and the runs that are then not in order, too rare or too short for the sample, are sorted by
+// themselves (k_order, k_runs).  Of kSampleShare sqrt(n) keys, s of n which lie in runs of one high part of
+// r keys make about kSampleShare^2 r s / (2 n) pairs of one run, so those are a few per cent of the keys or
+// less, and no longer than about sqrt(n) / 2.  All of it is decided on the device: the sort stays asynchronous.
+// 63-bit keys of 30-bit cells: 15,074,927 in 1,213 us with every pass, 777 now; 4 M 403 and 265, 2.1 M 283 and
+// 181.  Keys whose few low digits the high ones don't decide, 15,074,927: a tag of two bits beside keys that come
+// up twice 1,187 and 1,161; eleven low parts at random 1,213 and 935 (2,141 and 1,819 where every pass ran again
+// after the check).  Keys that fill their digits pay for the launches that find nothing to do, 15 us or so, which the
+// rule keeps to sorts that are long beside it: 4 M take 440, 1.5 M without the plan 250.
+constexpr size_t kSampleShare = 16;
 constexpr size_t kPlannedSort = 2u << 20;
 constexpr int kPlannedPasses = 6;
 
@@ -424,15 +551,23 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
     constexpr size_t smem = onesweep_smem<kThreads, kBits, kItems>();
     constexpr bool kCanPlan = kItems == kLargeItems;
     const bool planned = kCanPlan && n >= kPlannedSort && passes >= kPlannedPasses;
-    constexpr int kPlannedMode = kCanPlan ? 1 : 0, kLateMode = kCanPlan ? 2 : 0;  // only large tiles have these modes
-    const auto kernel = planned ? k_onesweep<kThreads, kBits, kItems, kPlannedMode> : k_onesweep<kThreads, kBits, kItems, 0>;
-    const auto late = k_onesweep<kThreads, kBits, kItems, kLateMode>;
+    const auto kernel = planned ? k_onesweep<kThreads, kBits, kItems, kCanPlan> : k_onesweep<kThreads, kBits, kItems, false>;
     FL_TRY_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                 "sort shared memory");
     unsigned hb = fl_blocks(n, 256, ctx->num_sms * 4);
+    // the sample's table, at most a quarter full, in the alternate keys
+    const size_t samples = std::max(kSampleShare * (size_t)std::sqrt((double)n), n / 256);
+    int lg = 0;
+    while ((1ull << lg) < 4 * samples) ++lg;
+    const uint64_t mask = range_mask(begin_bit, end_bit);
     (planned ? k_histogram<kBits, true> : k_histogram<kBits, false>)<<<hb, 256, 0, ctx->stream>>>(
-        keys, n, begin_bit, end_bit, passes, hist, plan);
+        keys, n, begin_bit, end_bit, passes, hist, plan, kalt, (size_t)1 << lg);
     FL_CHECK_LAUNCH(ctx, "k_histogram");
+    if (planned) {
+        k_sample<kBits><<<(unsigned)((samples + 255) / 256), 256, 0, ctx->stream>>>(keys, n, begin_bit, mask, samples,
+                                                                                    (unsigned long long*)kalt, lg, plan);
+        FL_CHECK_LAUNCH(ctx, "k_sample");
+    }
     cudaLaunchAttribute early{};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
@@ -446,35 +581,25 @@ int sort_passes(fl_ctx* ctx, uint64_t* keys, uint32_t* vals, size_t n, int begin
     uint64_t* ks[2] = {keys, kalt};
     uint32_t* vs[2] = {vals, valt};
     int cur = 0;  // of a planned sort the kernels work out the buffers
-    auto launch = [&](decltype(kernel) k, int ps) -> int {
+    for (int ps = 0; ps < passes; ++ps) {
         uint32_t* status = (uint32_t*)(stat0 + ps * stat_stride);
         unsigned* ticket = (unsigned*)(status + tiles * R);
         int sh = begin_bit + kBits * ps;
         const uint32_t* offs = hist + ps * R;
-        cudaLaunchKernelEx(&cfg, k, ks[cur], vs[cur], ks[cur ^ 1], vs[cur ^ 1], n, sh, digit_mask(end_bit, sh, kBits), offs,
-                           status, ticket, ctx->dev_status, (const SortPlan*)plan, ps, passes);
+        cudaLaunchKernelEx(&cfg, kernel, ks[cur], vs[cur], ks[cur ^ 1], vs[cur ^ 1], n, sh, digit_mask(end_bit, sh, kBits),
+                           offs, status, ticket, ctx->dev_status, (const SortPlan*)plan, ps);
         FL_CHECK_LAUNCH(ctx, "k_onesweep");
         if (!planned) cur ^= 1;
-        return FL_OK;
-    };
-    for (int ps = 0; ps < passes; ++ps) {
-        const int rc = launch(kernel, ps);
-        if (rc) return rc;
     }
     if (planned) {
         const unsigned grid = fl_blocks(n, 256, ctx->num_sms * 8);
-        k_order<<<grid, 256, 0, ctx->stream>>>(keys, kalt, n, plan, passes, begin_bit,
-                                               end_bit - begin_bit >= 64 ? ~0ull : (1ull << (end_bit - begin_bit)) - 1);
+        // over the status words, which the passes no longer need: passes * status_stride_min(n) >= 4 n bytes
+        uint32_t* list = (uint32_t*)stat0;
+        k_order<kBits><<<grid, 256, 0, ctx->stream>>>(keys, kalt, n, plan, passes, begin_bit, mask, list);
         FL_CHECK_LAUNCH(ctx, "k_order");
-        k_status_clear<<<ctx->num_sms, 256, 0, ctx->stream>>>(plan, (uint4*)stat0, passes * stat_stride / 16);
-        FL_CHECK_LAUNCH(ctx, "k_status_clear");
-        FL_TRY_CUDA(ctx, cudaFuncSetAttribute(late, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "sort shared memory");
-        cfg.gridDim = dim3((unsigned)ctx->num_sms * (kThreads == 512 ? 2 : (kBits == 8 ? 4 : 3)));
-        for (int ps = 0; ps < passes; ++ps) {
-            const int rc = launch(late, ps);
-            if (rc) return rc;
-        }
+        k_runs<kBits><<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(keys, vals, kalt, valt, n, plan, passes, begin_bit, mask,
+                                                                 list);
+        FL_CHECK_LAUNCH(ctx, "k_runs");
         k_home<<<grid, 256, 0, ctx->stream>>>(keys, vals, kalt, valt, n, plan, passes);
         FL_CHECK_LAUNCH(ctx, "k_home");
     }
