@@ -335,9 +335,10 @@ __device__ __forceinline__ uint32_t sibling_in_run(const fl_probe& P, const fl_m
     *ok = false;
     if (i < (size_t)h) return FL_INVALID_INDEX;
     const size_t j = i - h + c;
-    if (j >= m.n || m.level[j] != l || digit(j) != c || (m.x[j] >> 1) != (m.x[i] >> 1) || (m.y[j] >> 1) != (m.y[i] >> 1) ||
-        (m.z[j] >> 1) != (m.z[i] >> 1) || (m.case_id && m.case_id[j] != m.case_id[i]))
-        return FL_INVALID_INDEX;
+    if (j >= m.n) return FL_INVALID_INDEX;
+    const bool same = (m.level[j] == l) & (digit(j) == c) & ((m.x[j] >> 1) == (m.x[i] >> 1)) &
+                      ((m.y[j] >> 1) == (m.y[i] >> 1)) & ((m.z[j] >> 1) == (m.z[i] >> 1));  // loads side by side
+    if (!same || (m.case_id && m.case_id[j] != m.case_id[i])) return FL_INVALID_INDEX;
     *ok = m.flags[j] == -1 && m.state[j] == 0;
     return (uint32_t)j;
 }
