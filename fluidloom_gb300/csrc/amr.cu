@@ -1138,12 +1138,13 @@ int fl_neighbour_rebuild(fl_ctx* ctx, const fl_mesh* mesh, const fl_adapt_config
     fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material, mesh->case_id, n};
     const int32_t ext[3] = {std::max(cfg->ext[0], 1), std::max(cfg->ext[1], 1), std::max(cfg->ext[2], 1)};
     bool done = false;
-    rc = fl_neighbours_octree(ctx, md, dom, ext, subslots, cv.p, nbr, &done);
+    int deepest;
+    rc = fl_neighbours_octree(ctx, md, dom, ext, subslots, cv.p, nbr, &done, &deepest);
     if (rc) return rc;
     if (done) return FL_OK;
     uint32_t* marks = cv.take<uint32_t>(n);
     fl_locator L;
-    rc = fl_locator_build(ctx, md, dom, cv.p, &L);
+    rc = fl_locator_build(ctx, md, dom, cv.p, &L, deepest);
     if (rc) return rc;
     rc = fl_neighbours_sorted(ctx, md, dom, L, subslots, nbr, marks);
     if (rc) return rc;

@@ -232,13 +232,14 @@ int fl_neighbours_sorted(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev&
 
 // The same rows for a single-case mesh through an octree of its leaves (ext: level-0 cells per
 // axis), with no sort and no key order wanted.  *done is false, and the rows undefined, when the
-// mesh has no such octree -- leaves that overlap or lie outside the domain, a gap at a node's lowest
-// corner, a domain far larger than the leaves, levels far apart or deeper than dom.max_level -- and
-// the sorted locator must serve it.  scratch: fl_neighbours_octree_scratch(n) bytes; synchronises and
-// collects the device status.
+// mesh has no such octree -- leaves that overlap or lie outside the domain, gaps so many that its nodes
+// are more than a quarter of its leaves, a domain far larger than the leaves, levels far apart or deeper than
+// dom.max_level -- and the sorted locator must serve it; *deepest is then the deepest leaf level, -1 if it
+// was not looked for.  scratch: fl_neighbours_octree_scratch(n) bytes; synchronises and collects the
+// device status.
 size_t fl_neighbours_octree_scratch(size_t n);
 int fl_neighbours_octree(fl_ctx* ctx, const fl_mesh_dev& m, const fl_domain_dev& dom, const int32_t* ext, int subslots,
-                         void* scratch, uint32_t* nbr, bool* done);
+                         void* scratch, uint32_t* nbr, bool* done, int* deepest);
 
 int fl_hash_lg(uint64_t cap);
 uint64_t fl_table_capacity(size_t n);
