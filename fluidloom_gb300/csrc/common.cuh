@@ -25,7 +25,7 @@ struct fl_ctx {
     uint32_t* dev_status = nullptr;     // device-side status words (see FL_DEVSTAT_*)
     uint32_t* host_status = nullptr;    // pinned mirror
     char* host_read = nullptr;          // pinned landing area of small reads (kHostReadBytes)
-    cudaMemPool_t pool = nullptr;       // stream-ordered allocations (fl_dev_malloc_async)
+    cudaMemPool_t pool = nullptr;       // stream-ordered allocations (fl_dev_malloc_async); the device's
     std::string last_error;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // fl_ctx_timer_start / stop
     void* soa = nullptr;                       // structure-of-arrays field manager (fields.cu)

@@ -3,6 +3,8 @@
 
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 int fl_set_error(fl_ctx* ctx, int code, const std::string& msg) {
     if (ctx) ctx->last_error = msg;
@@ -29,7 +31,7 @@ cudaError_t fl_dev_malloc(fl_ctx* ctx, void** p, size_t bytes) {
     *p = nullptr;
     if (injected_alloc_failure(ctx)) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && ctx && ctx->pool) {  // with what the context's pool keeps free
+    if (e == cudaErrorMemoryAllocation && ctx && ctx->pool) {  // with what the device's pool keeps free
         cudaGetLastError();
         cudaStreamSynchronize(ctx->stream);
         cudaMemPoolTrimTo(ctx->pool, 0);
@@ -102,25 +104,56 @@ int fl_collect_device_status(fl_ctx* ctx, const char* what) {
     return FL_OK;
 }
 
-// The context's own memory pool.  CUDA's default pool hands every free block back to the system
+// The memory pool of a device's contexts.  CUDA's default pool hands every free block back to the system
 // whenever a stream is synchronised, so a regrid, which replaces its mesh's columns, mapped and
 // unmapped them each time (a 25 M-leaf regrid 9,180 -> 7,680 us, with the small reads through pinned
-// memory); this one keeps up to a 64th of the device's memory between calls and gives all of it
-// back with the context, or when an allocation would fail for want of it.
-static int create_pool(fl_ctx* c) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = c->device;
-    if (cudaMemPoolCreate(&c->pool, &props) != cudaSuccess) {
-        c->pool = nullptr;
-        return FL_E_OOM;
+// memory); this one keeps up to a 64th of the device's memory between calls, all contexts together, and
+// gives it back when an allocation of any of them would fail for want of it, and with the last
+// context.  Other users of the device find that much less free meanwhile.
+namespace {
+struct DevicePool {
+    cudaMemPool_t pool;
+    int users;
+};
+std::mutex g_pools_lock;
+std::map<int, DevicePool>& device_pools() {
+    static auto* pools = new std::map<int, DevicePool>;  // contexts may outlive the statics of an exiting process
+    return *pools;
+}
+}  // namespace
+
+static int acquire_pool(fl_ctx* c) {
+    std::lock_guard<std::mutex> hold(g_pools_lock);
+    auto it = device_pools().find(c->device);
+    if (it == device_pools().end()) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->device;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return FL_E_OOM;
+        size_t free_b = 0, total_b = 0;
+        uint64_t keep = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess ? total_b / 64 : 0;
+        if (!keep || cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return FL_E_CUDA;
+        }
+        it = device_pools().emplace(c->device, DevicePool{pool, 0}).first;
     }
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return FL_E_CUDA;
-    uint64_t keep = total_b / 64;
-    return cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess ? FL_OK : FL_E_CUDA;
+    ++it->second.users;
+    c->pool = it->second.pool;
+    return FL_OK;
+}
+
+static void release_pool(fl_ctx* c) {
+    std::lock_guard<std::mutex> hold(g_pools_lock);
+    const auto it = device_pools().find(c->device);
+    if (--it->second.users == 0) {
+        cudaMemPoolDestroy(it->second.pool);  // allocations still in use stay valid until they are freed
+        device_pools().erase(it);
+    }
+    c->pool = nullptr;
 }
 
 extern "C" {
@@ -164,7 +197,7 @@ int fl_ctx_create(int device, fl_ctx** out) {
     if (rc == FL_OK && cudaMemset(c->dev_status, 0, FL_DEVSTAT_WORDS * 4) != cudaSuccess) rc = FL_E_CUDA;
     if (rc == FL_OK && cudaMallocHost(&c->host_status, FL_DEVSTAT_WORDS * 4) != cudaSuccess) rc = FL_E_OOM;
     if (rc == FL_OK && cudaMallocHost(&c->host_read, kHostReadBytes) != cudaSuccess) rc = FL_E_OOM;
-    if (rc == FL_OK) rc = create_pool(c);
+    if (rc == FL_OK) rc = acquire_pool(c);
     if (rc != FL_OK) {
         cudaGetLastError();
         fl_ctx_destroy(c);
@@ -182,7 +215,7 @@ int fl_ctx_destroy(fl_ctx* ctx) {
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->host_status) cudaFreeHost(ctx->host_status);
     if (ctx->host_read) cudaFreeHost(ctx->host_read);
-    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);  // allocations still in use stay valid until they are freed
+    if (ctx->pool) release_pool(ctx);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
