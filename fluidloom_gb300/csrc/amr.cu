@@ -133,9 +133,45 @@ __global__ void k_shadow_update(fl_mesh_dev m, int mode, int max_level, uint8_t*
     }
 }
 
-// detect_balance_violations (balance_enforce.cl:57-147), exact lookups.  Eight lanes a leaf, a face
-// each on six of them, so that a leaf's lookups -- a key encoding and a random table slot per level
-// tried -- overlap instead of following one another (67,000 leaves: a thread a leaf 38 us, 20 now).
+// detect_balance_violations (balance_enforce.cl:57-147), exact lookups: a leaf, and whether the one across
+// its face f ends two or more levels above it.
+struct Face6 {
+    const fl_domain_dev::Case* d;
+    int64_t at[3], size;
+    uint16_t cs;
+    int level;
+};
+__device__ __forceinline__ Face6 face6_of(const fl_mesh_dev& m, const fl_domain_dev& dom,
+                                          const uint8_t* __restrict__ shadow, size_t i) {
+    Face6 L;
+    L.cs = m.case_id ? m.case_id[i] : 0;
+    L.d = dom.c + L.cs;
+    L.level = shadow[i];
+    const int sh = dom.anchor_level - m.level[i], ex = dom.anchor_level - L.level;
+    L.size = ex > 0 ? ((int64_t)1 << ex) : 1;
+    L.at[0] = (int64_t)m.x[i] << sh;
+    L.at[1] = (int64_t)m.y[i] << sh;
+    L.at[2] = (int64_t)m.z[i] << sh;
+    return L;
+}
+__device__ __forceinline__ bool face6_hit(const Face6& L, bool has_case, const fl_domain_dev& dom, const KeyTables& T,
+                                          const uint64_t* __restrict__ tk, int lg, const uint8_t* __restrict__ shadow,
+                                          int f) {
+    const int64_t move = (f & 1) ? L.size : -1;
+    int64_t p[3] = {L.at[0] + (f < 2 ? move : 0), L.at[1] + ((f >> 1) == 1 ? move : 0), L.at[2] + (f > 3 ? move : 0)};
+    if (!fold3(p, *L.d, dom.anchor_level)) return false;
+    const uint32_t r = fl_locate(T.t1, T.t3, tk, nullptr, lg, shadow, dom, L.cs, has_case, p, L.level);
+    return r != FL_INVALID_INDEX && (int)shadow[r] > L.level + 1;
+}
+
+// kSpread: eight lanes a leaf, a face each on six of them, so that a leaf's lookups -- a key encoding and a
+// random table slot per level tried -- overlap instead of following one another.  Otherwise a thread a
+// leaf, its faces in turn, which takes fewer instructions and has neighbouring leaves probe one face
+// together.  Spread and not, us, balanced meshes: 28,323 leaves 49 and 73 (two rounds), 56,253 19.5 and 26.3,
+// 81,649 56 and 60 (two), 281,121 48 and 38, 2,859,648 491 and 312; 16.8 M on one level 3,190 and 2,300.  (The
+// faces unrolled, six copies of the search: 81 on 7,302 leaves for 55.)
+constexpr size_t kSpreadLeaves = 1u << 17;
+template <bool kSpread>
 __global__ void __launch_bounds__(kT) k_detect_face6(fl_mesh_dev m, fl_domain_dev dom, const uint64_t* __restrict__ tk,
                                                      int lg, const uint8_t* __restrict__ shadow,
                                                      uint8_t* __restrict__ viol,
@@ -143,33 +179,31 @@ __global__ void __launch_bounds__(kT) k_detect_face6(fl_mesh_dev m, fl_domain_de
     __shared__ KeyTables T;
     fl_keys_fill_tables(T.t1, T.t3, false);
     __syncthreads();
-    const int lane = threadIdx.x & 31, f = lane & 7;
-    const size_t step = (size_t)gridDim.x * (blockDim.x >> 3);
     uint32_t local = 0;
-    for (size_t i0 = (size_t)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 5) * 4; i0 < m.n; i0 += step) {
-        const size_t i = i0 + (lane >> 3);
-        bool hit = false;
-        if (i < m.n && f < 6 && m.state[i] == 0) {
-            const uint16_t cs = m.case_id ? m.case_id[i] : 0;
-            const fl_domain_dev::Case& d = dom.c[m.case_id ? cs : 0];
-            const int sl = shadow[i];
-            const int sh = dom.anchor_level - m.level[i];
-            const int ex = dom.anchor_level - sl;
-            const int64_t ss = ex > 0 ? ((int64_t)1 << ex) : 1;
-            int64_t p[3] = {(int64_t)m.x[i] << sh, (int64_t)m.y[i] << sh, (int64_t)m.z[i] << sh};
-            const int64_t move = (f & 1) ? ss : -1;
-            if ((f >> 1) == 0) p[0] += move;
-            else if ((f >> 1) == 1) p[1] += move;
-            else p[2] += move;
-            if (fold3(p, d, dom.anchor_level)) {
-                const uint32_t r = fl_locate(T.t1, T.t3, tk, nullptr, lg, shadow, dom, cs, m.case_id != nullptr, p, sl);
-                hit = r != FL_INVALID_INDEX && (int)shadow[r] > sl + 1;
+    if (kSpread) {
+        const int lane = threadIdx.x & 31, f = lane & 7;
+        const size_t step = (size_t)gridDim.x * (blockDim.x >> 3);
+        for (size_t i0 = (size_t)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 5) * 4; i0 < m.n; i0 += step) {
+            const size_t i = i0 + (lane >> 3);
+            const bool hit = i < m.n && f < 6 && m.state[i] == 0 &&
+                             face6_hit(face6_of(m, dom, shadow, i), m.case_id != nullptr, dom, T, tk, lg, shadow, f);
+            const unsigned faces = (__ballot_sync(0xFFFFFFFFu, hit) >> (lane & 24)) & 0xFFu;
+            if (f == 0 && i < m.n) {
+                viol[i] = faces ? 1 : 0;
+                local += faces ? 1u : 0u;
             }
         }
-        const unsigned faces = (__ballot_sync(0xFFFFFFFFu, hit) >> (lane & 24)) & 0xFFu;
-        if (f == 0 && i < m.n) {
-            viol[i] = faces ? 1 : 0;
-            local += faces ? 1u : 0u;
+    } else {
+        const size_t step = (size_t)gridDim.x * blockDim.x;
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < m.n; i += step) {
+            bool hit = false;
+            if (m.state[i] == 0) {
+                const Face6 L = face6_of(m, dom, shadow, i);
+#pragma unroll 1
+                for (int f = 0; f < 6 && !hit; ++f) hit = face6_hit(L, m.case_id != nullptr, dom, T, tk, lg, shadow, f);
+            }
+            viol[i] = hit ? 1 : 0;
+            local += hit ? 1u : 0u;
         }
     }
     if (local) atomicAdd(count, local);
@@ -898,8 +932,11 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
         uint32_t* list = (act && mode == 1 && (it > 0 || first_listed)) ? (uint32_t*)(act + fl_align256(md.n)) : nullptr;
         uint32_t* list_n = counters + 4;  // free until the merge grouping after balance
         if (mode == 0) {
-            k_detect_face6<<<fl_blocks(md.n * 8, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(md, dom, tk, lg, shadow, viol,
-                                                                                       counters);
+            if (md.n <= kSpreadLeaves)
+                k_detect_face6<true><<<fl_blocks(md.n * 8, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(
+                    md, dom, tk, lg, shadow, viol, counters);
+            else
+                k_detect_face6<false><<<nb, kT, 0, ctx->stream>>>(md, dom, tk, lg, shadow, viol, counters);
         } else {
             k_clear_u8<<<nb, kT, 0, ctx->stream>>>(viol, md.n);
             if (list) {
