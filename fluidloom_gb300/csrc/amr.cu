@@ -75,19 +75,20 @@ __device__ __forceinline__ uint8_t shadow_of(const fl_mesh_dev& m, size_t i, int
 
 // Shadow levels; lowest[0] / lowest[1] (when given) receive their minimum and
 // maximum; refining (when given) a byte per leaf, set where the leaf will split.
-// FULL26 takes four leaves a thread where the columns' addresses allow it (25 M
-// leaves, 7 bytes each: 73 us, 40 now).
+// Four leaves a thread where the columns' addresses allow it (25 M leaves, 7
+// bytes each: 73 us, 40 now; 16.8 M for FACE6, 2 bytes each: 52 us, 23 now).
 __global__ void k_shadow(fl_mesh_dev m, int mode, int max_level, uint8_t* __restrict__ shadow,
                          uint32_t* __restrict__ lowest, uint8_t* __restrict__ refining) {
     size_t stride = (size_t)gridDim.x * blockDim.x;
     unsigned lo = 255u, hi = 0u;
     const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool quads = mode == 1 && ((uintptr_t)m.flags & 15) == 0 &&
+    const bool quads = (mode == 0 || ((uintptr_t)m.flags & 15) == 0) &&
                        (((uintptr_t)m.level | (uintptr_t)m.state | (uintptr_t)shadow | (uintptr_t)refining) & 3) == 0;
     const size_t nq = quads ? m.n / 4 : 0;
     for (size_t q = t0; q < nq; q += stride) {
-        const int4 f = ((const int4*)m.flags)[q];
-        const uint32_t lv = ((const uint32_t*)m.level)[q], st = ((const uint32_t*)m.state)[q];
+        const uint32_t lv = ((const uint32_t*)m.level)[q];
+        const int4 f = mode == 0 ? make_int4(0, 0, 0, 0) : ((const int4*)m.flags)[q];
+        const uint32_t st = mode == 0 ? 0u : ((const uint32_t*)m.state)[q];
         const int fl[4] = {f.x, f.y, f.z, f.w};
         uint32_t up = 0;
         for (int k = 0; k < 4; ++k) {
