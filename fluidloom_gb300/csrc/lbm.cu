@@ -1560,8 +1560,14 @@ __global__ void k_blob_flags(fl_mesh_dev m, const float* __restrict__ blobs, int
 //   + 2 n 2^-24 v (rounding of both sums, whose terms are >= 0),
 // and the kernel allows e0 = 4e-6 A and e1 = 1.5e-7 n per v: a cell whose sum lies that close to a
 // threshold (one in a few thousand) is worked out again by the exact sum, so the flags are the same.
-// Bound by instruction issue: 25 M leaves, 48 blobs, 1,370 -> 372 us.
+// Bound by instruction issue: 25 M leaves, 48 blobs, 1,370 -> 372 us.  Taken from kNearCells cells and
+// kNearBlobs blobs on; below, its four cells a thread leave the GPU idle, or the exact sum is short
+// beside the columns.  Exact and near, us: 64,000 cells, 12 blobs 3.6 and 4.6, 48 blobs 8.2 and 10.3; 125,000 cells,
+// 12 blobs 4.9 and 4.8; 262,144 cells, 4 blobs 3.8 and 3.7; 16.8 M cells, 1 blob 78 and 104, 3 blobs 109 and
+// 110, 4 blobs 130 and 112.
 constexpr int kBlobCells = 4;
+constexpr size_t kNearCells = 1u << 17;
+constexpr int kNearBlobs = 4;
 
 __global__ void __launch_bounds__(256) k_blob_flags_near(fl_mesh_dev m, const float* __restrict__ blobs, int nblobs,
                                                          float lo, float hi, int max_level, float e0, float e1,
@@ -1639,7 +1645,8 @@ extern "C" int fl_flags_from_blobs(fl_ctx* ctx, fl_mesh* mesh, const float* blob
     fl_mesh_dev md{mesh->x, mesh->y, mesh->z, mesh->level, mesh->state, mesh->flags, mesh->material, mesh->case_id,
                    mesh->num_cells};
     // the near sum's bound holds for decaying blobs of amplitude >= 0 around the unit cube
-    bool near = lo > -1e30f && lo < 1e30f && hi > -1e30f && hi < 1e30f;
+    bool near = mesh->num_cells >= kNearCells && nblobs >= kNearBlobs && lo > -1e30f && lo < 1e30f && hi > -1e30f &&
+                hi < 1e30f;
     double amps = 0.0;
     for (int k = 0; k < nblobs; ++k) {
         const float* B = blobs_host + 5 * k;
