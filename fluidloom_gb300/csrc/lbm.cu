@@ -1477,7 +1477,9 @@ __global__ void __launch_bounds__(4 * kChunkBricks) k_chunk_sums(const float* __
         }
         red[threadIdx.x] = acc;
         __syncthreads();
-        for (int o = 2 * kChunkBricks; o >= 4; o >>= 1) {
+        int o = 2 * kChunkBricks;
+        while (o >= 4 && (uint32_t)o >= 4u * (r.y - r.x)) o >>= 1;  // only zeros up there
+        for (; o >= 4; o >>= 1) {
             if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
             __syncthreads();
         }
@@ -1486,16 +1488,33 @@ __global__ void __launch_bounds__(4 * kChunkBricks) k_chunk_sums(const float* __
     }
 }
 
-// A warp per case and component: its chunks' sums, lane by lane in chunk order, then a fixed tree.
+// Per case and component its chunks' sums, lane by lane in chunk order, then a fixed tree: a warp takes `per`
+// (1 or 32) of them, those of at most four chunks a lane each (in the tree's order), the others one after
+// another.  A warp each (per = 1) but for many cases of few chunks: 4,096 cases of a brick took 8.2 us that way, 2.4
+// with a thread each and its chunks in turn, 2.6 now.
 __global__ void k_case_sums(const double* __restrict__ chunk_part, const uint32_t* __restrict__ case_chunk,
-                            int ncases, double* __restrict__ out) {
-    const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (t >= ncases * 4) return;
-    const int cs = t >> 2, k = t & 3;
-    double s = 0.0;
-    for (uint32_t c = case_chunk[cs] + lane; c < case_chunk[cs + 1]; c += 32) s += chunk_part[(size_t)c * 4 + k];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if (lane == 0) out[t] = s;
+                            int ncases, int per, double* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int first = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
+    const int mine = first + lane;
+    bool more = false;
+    if (lane < per && mine < ncases * 4) {
+        const uint32_t c = case_chunk[mine >> 2], n = case_chunk[(mine >> 2) + 1] - c;
+        const double* v = chunk_part + (size_t)c * 4 + (mine & 3);
+        more = n > 4;
+        if (!more) {
+            double s[4];
+            for (uint32_t j = 0; j < 4; ++j) s[j] = j < n ? 0.0 + v[4 * j] : 0.0;
+            out[mine] = (s[0] + s[2]) + (s[1] + s[3]);
+        }
+    }
+    for (unsigned m = __ballot_sync(0xFFFFFFFFu, more); m; m &= m - 1) {
+        const int t = first + __ffs(m) - 1, cs = t >> 2, k = t & 3;
+        double s = 0.0;
+        for (uint32_t c = case_chunk[cs] + lane; c < case_chunk[cs + 1]; c += 32) s += chunk_part[(size_t)c * 4 + k];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        if (lane == 0) out[t] = s;
+    }
 }
 
 // exp(x) for x <= 0 from the mathematics: x = n ln2 + r with |r| <= ln2/2
@@ -2897,7 +2916,8 @@ int fl_pool_conservation_async(fl_ctx* ctx, fl_pool* P, double* out) {
             P->part, P->mesh.level, P->d_chunks, P->nchunks, P->chunk_part);
         FL_CHECK_LAUNCH(ctx, "k_chunk_sums");
     }
-    k_case_sums<<<(nc * 4 + 7) / 8, 256, 0, ctx->stream>>>(P->chunk_part, P->d_case_chunk, nc, P->cons);
+    const int per = nc >= 256 && P->nchunks <= 4u * (uint32_t)nc ? 32 : 1;
+    k_case_sums<<<(nc * 4 / per + 8) / 8, 256, 0, ctx->stream>>>(P->chunk_part, P->d_case_chunk, nc, per, P->cons);
     FL_CHECK_LAUNCH(ctx, "k_case_sums");
     FL_TRY_CUDA(ctx, cudaMemcpyAsync(out, P->cons, nc * 32, cudaMemcpyDefault, ctx->stream), "conservation");
     return FL_OK;
