@@ -38,7 +38,9 @@ __global__ void k_hash_clear(uint64_t* __restrict__ tk, uint32_t* __restrict__ t
 // plain store; a thread that finds its key already there flags the build
 // (FL_DEVSTAT_HASH_DUPS) and stores nothing.  Without repeated keys that is
 // the table; with them the passes below give each repeated key the value
-// of its last input.
+// of its last input.  kIndex: the values are the input indices, whose maximum (FL_INVALID_INDEX
+// is -1 there) is the last input's at once.
+template <bool kIndex>
 __global__ void __launch_bounds__(256) k_hash_insert(uint64_t* __restrict__ tk, uint32_t* __restrict__ tv, int lg,
                                                      const uint64_t* __restrict__ keys,
                                                      const uint32_t* __restrict__ vals, size_t n,
@@ -53,8 +55,12 @@ __global__ void __launch_bounds__(256) k_hash_insert(uint64_t* __restrict__ tk, 
         int p = 0;
         for (; p < kProbeLimit; ++p) {
             const unsigned long long prev = atomicCAS((unsigned long long*)(tk + s), FL_EMPTY_KEY, k);
-            if (prev == FL_EMPTY_KEY) tv[s] = vals ? vals[i] : (uint32_t)i;
-            if (prev == k) dup = true;
+            if (kIndex) {
+                if (prev == FL_EMPTY_KEY || prev == k) atomicMax((int*)(tv + s), (int)i);
+            } else {
+                if (prev == FL_EMPTY_KEY) tv[s] = vals ? vals[i] : (uint32_t)i;
+                if (prev == k) dup = true;
+            }
             if (prev == FL_EMPTY_KEY || prev == k) break;
             s = (s + 1) & mask;
         }
@@ -911,16 +917,18 @@ int fl_hash_build(fl_ctx* ctx, uint64_t* table_keys, uint32_t* table_vals, uint6
     if (!table_keys || !table_vals || capacity == 0 || (capacity & (capacity - 1)) || (n && !keys))
         return fl_set_error(ctx, FL_E_INVALID_ARG, "fl_hash_build: bad table or capacity not a power of two");
     if (n > capacity) return fl_set_error(ctx, FL_E_CAPACITY, "fl_hash_build: more keys than slots");
-    FL_TRY_CUDA(ctx, cudaMemsetAsync(ctx->dev_status + FL_DEVSTAT_HASH_DUPS, 0, 4, ctx->stream), "hash flag");
+    const bool index = !vals && n < (1ull << 31);  // as int
+    if (!index)
+        FL_TRY_CUDA(ctx, cudaMemsetAsync(ctx->dev_status + FL_DEVSTAT_HASH_DUPS, 0, 4, ctx->stream), "hash flag");
     k_hash_clear<<<fl_blocks(capacity, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(table_keys, table_vals, capacity);
     FL_CHECK_LAUNCH(ctx, "k_hash_clear");
     if (n) {
-        k_hash_insert<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+        (index ? k_hash_insert<true> : k_hash_insert<false>)<<<fl_blocks(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
             table_keys, table_vals, fl_hash_lg(capacity), keys, vals, n, ctx->dev_status);
         FL_CHECK_LAUNCH(ctx, "k_hash_insert");
     }
     int rc = fl_collect_device_status(ctx, "fl_hash_build");
-    if (rc || !ctx->host_status[FL_DEVSTAT_HASH_DUPS]) return rc;
+    if (rc || index || !ctx->host_status[FL_DEVSTAT_HASH_DUPS]) return rc;
     // repeated keys: the winner of each slot in a second round
     rc = fl_scratch_reserve(ctx, capacity * 4);
     if (rc) return rc;
@@ -931,7 +939,8 @@ int fl_hash_build(fl_ctx* ctx, uint64_t* table_keys, uint32_t* table_vals, uint6
     FL_CHECK_LAUNCH(ctx, "k_hash_dup_winners");
     k_hash_dup_values<<<fl_blocks(capacity, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(table_vals, win, vals, capacity);
     FL_CHECK_LAUNCH(ctx, "k_hash_dup_values");
-    return fl_collect_device_status(ctx, "fl_hash_build");
+    FL_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "fl_hash_build");  // neither pass has a status to report
+    return FL_OK;
 }
 
 int fl_hash_query(fl_ctx* ctx, const uint64_t* table_keys, const uint32_t* table_vals, uint64_t capacity,
