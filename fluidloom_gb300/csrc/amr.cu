@@ -931,7 +931,7 @@ int fl_balance_run(fl_ctx* ctx, fl_mesh_dev md, int32_t* flags, const fl_domain_
         // this round's probing leaves (all of them in the first round) and the next round's
         uint8_t* nxt = (act && mode == 1) ? act : nullptr;
         uint32_t* list = (act && mode == 1 && (it > 0 || first_listed)) ? (uint32_t*)(act + fl_align256(md.n)) : nullptr;
-        uint32_t* list_n = counters + 4;  // free until the merge grouping after balance
+        uint32_t* list_n = counters + 4;
         if (mode == 0) {
             if (md.n <= kSpreadLeaves)
                 k_detect_face6<true><<<fl_blocks(md.n * 8, kT, ctx->num_sms * 8), kT, 0, ctx->stream>>>(

@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev d
         }
     }
     bad = __reduce_or_sync(0xFFFFFFFFu, bad);
-    if (bad && lane == 0) atomicOr(order, bad);
+    if (lane == 0 && (bad & ~*(volatile uint32_t*)order)) atomicOr(order, bad);  // once, nearly
 }
 
 __global__ void k_iota(uint32_t* __restrict__ ids, size_t n) {
