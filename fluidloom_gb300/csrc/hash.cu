@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(256) k_level_range(const uint8_t* __restrict__
 // id above bit 3 * (depth - cut)).
 //
 // order (when given) gets bit 0 when some run start is smaller than the one
-// before it, bit 1 when some is the same (a leaf listed twice, or overlapping leaves).  A warp takes a range of consecutive leaves and keeps the last of
+// before it, bit 1 when some is the same (a leaf listed twice, or overlapping
+// leaves).  A warp takes a range of consecutive leaves and keeps the last of
 // 32 for the next 32, so only the start of its range is encoded twice (25 M
 // leaves: 107 us and a pass of 41 over the keys, 135 now).
 __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev dom, int cut,
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(256) k_run_keys(fl_mesh_dev m, fl_domain_dev d
         }
     }
     bad = __reduce_or_sync(0xFFFFFFFFu, bad);
-    if (lane == 0 && (bad & ~*(volatile uint32_t*)order)) atomicOr(order, bad);  // once, nearly
+    if (bad && lane == 0) atomicOr(order, bad);  // (bad is 0 where order is not given)
 }
 
 __global__ void k_iota(uint32_t* __restrict__ ids, size_t n) {
